@@ -33,6 +33,7 @@ PER_FILE = {"ic_pipeline.cu": ["--fmad=false"]}
 CXX_FLAGS = ["-O2", "-fPIC", "-std=c++17", "-Wall", "-I" + CSRC, "-I" + INC]
 
 CU_SOURCES = ["step_engine.cu", "batch_engine.cu", "batch_fp64.cu", "batch_fp32.cu", "batch_mixed.cu",
+              "box_fp64.cu", "box_fp32.cu", "box_mixed.cu",
               "ic_pipeline.cu", "static_poisson.cu", "diagnostics.cu"]
 CPP_SOURCES = ["ifdm_api.cpp", "io.cpp", "snapshot_stream.cpp", "ic_stream.cpp"]
 

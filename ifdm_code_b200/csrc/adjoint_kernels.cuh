@@ -14,20 +14,9 @@
 #pragma once
 
 #include "step_kernels.cuh"
+#include "timestep.cuh"
 
 namespace ifdm {
-
-// Coefficients of one recorded step, as its passes used them.
-struct StepLog {
-    double coefP;        // kick coefficient of the stored phi
-    double coefQ;        // kick coefficient of |psi_s|^2
-    double alpha;        // dither phase of the kick
-    double drift_s;      // drift phase per unit kappa^2
-    double cre, cim;     // offset c of this step
-    double pendP, pendQ; // half kick owed after this step
-    double gphase;       // accumulated dither after this step's kick
-    double a, dt_KE, dt_PE, dt_QI;
-};
 
 // Load one recorded step into the pass state and rebuild its drift tables;
 // conj != 0 writes the conjugate tables (the adjoint drift) instead.
@@ -61,23 +50,7 @@ __global__ void k_replay_step(TState *__restrict__ ts, const StepLog *__restrict
 }
 
 // Append the step the timestep kernel just prepared to the log.
-__global__ void k_log_step(const TState *__restrict__ ts, StepLog *__restrict__ lg) {
-    StepLog e;
-    e.coefP = ts->coefP;
-    e.coefQ = ts->coefQ;
-    e.alpha = ts->alpha;
-    e.drift_s = ts->drift_s;
-    e.cre = ts->cre;
-    e.cim = ts->cim;
-    e.pendP = ts->pendP;
-    e.pendQ = ts->pendQ;
-    e.gphase = ts->gphase;
-    e.a = ts->a;
-    e.dt_KE = ts->dt_KE;
-    e.dt_PE = ts->dt_PE;
-    e.dt_QI = ts->dt_QI;
-    *lg = e;
-}
+__global__ void k_log_step(const TState *__restrict__ ts, StepLog *__restrict__ lg) { log_step(ts, lg); }
 
 // w = Im(conj(g') psi'), psi' = psi exp(-i theta), theta = a phi + b |psi|^2 + alpha
 template <typename R, typename K>

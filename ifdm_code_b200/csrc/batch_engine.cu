@@ -87,7 +87,9 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
     for (auto &c : cls_) {
         if (!K_->items(c.N, c.items, &c.smem)) return "batch: res " + std::to_string(c.N) + " is not a batch size";
         const size_t nb = c.boxes.size();
-        CUDA_TRY(cudaMalloc(&c.d_boxes, sizeof(BatchBox) * nb));
+        const BoxKernels &bk = box_kernels(precision_);
+        c.box = bk.fits(c.N);
+        CUDA_TRY(cudaMalloc(&c.d_boxes, std::max(sizeof(BatchBox), sizeof(BoxRun)) * nb));
         CUDA_TRY(cudaMalloc(&c.d_segs, sizeof(BatchSeg) * nb * kBatchPhases));
         CUDA_TRY(cudaMalloc(&c.d_ctr, sizeof(unsigned long long) * (nb + 1)));
         CUDA_TRY(cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
@@ -95,8 +97,17 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
         CUDA_TRY(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
         for (int v = 0; v < 2; ++v) {
             int fit = 0;
-            std::string e = K_->setup(c.N, v, c.smem, &fit);
+            std::string e = c.box ? K_->box_setup(c.N, v) : K_->setup(c.N, v, c.smem, &fit);
+            if (e.empty() && c.box) e = bk.setup(c.N, v);
             if (!e.empty()) return e;
+        }
+        if (c.box) {
+            // A cluster of 16 CTAs a box, all steps in one launch, while a CTA has
+            // at most two planes and every cluster is resident at once; else a
+            // launch per phase over all boxes (group 0).  FP32, us a step, one
+            // against the other: 8 boxes of 32^3 29 / 39, 32 of 48^3 154 / 133,
+            // 2 of 96^3 224 / 110, 64 of 16^3 46 / 38.
+            c.group = c.N <= 32 && bk.resident(c.N, 16, true) >= (int)nb ? 16 : 0;
         }
     }
     CUDA_TRY(cudaMalloc(&d_status_, sizeof(int)));
@@ -109,12 +120,29 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
 
 std::string BatchEngine::prepare(const double *dt_scale) {
     // box tables (the engines' views are read again: a state load may set new constants)
-    std::vector<std::vector<BatchBox>> hb(cls_.size());
+    std::vector<std::vector<unsigned char>> hb(cls_.size());
     std::vector<unsigned char> raw;
     for (size_t ci = 0; ci < cls_.size(); ++ci) {
         Class &c = cls_[ci];
         for (int b : c.boxes) {
             const EngineView v = boxes_[b]->view();
+            if (c.box) {
+                BoxRun x;
+                std::memset(&x, 0, sizeof x);
+                x.psi = v.psi;
+                x.phi = v.phi;
+                x.rhok = v.rhok;
+                x.tw = v.tw;
+                x.ts = v.ts;
+                x.scr = (BoxScratch *)v.box_scr;
+                x.ph = v.phys;
+                x.ph.dt_scale = dt_scale[b];
+                x.win_rows = v.win_rows;
+                x.win_tail = v.win_tail;
+                x.timestep = 1;
+                hb[ci].insert(hb[ci].end(), (const unsigned char *)&x, (const unsigned char *)&x + sizeof x);
+                continue;
+            }
             BatchBox x;
             std::memset(&x, 0, sizeof x);
             x.N = v.N;
@@ -137,9 +165,9 @@ std::string BatchEngine::prepare(const double *dt_scale) {
             }
             x.prefix[kBatchPhases] = acc;
             x.step_items = acc;
-            hb[ci].push_back(x);
-            raw.insert(raw.end(), (const unsigned char *)&x, (const unsigned char *)&x + sizeof x);
+            hb[ci].insert(hb[ci].end(), (const unsigned char *)&x, (const unsigned char *)&x + sizeof x);
         }
+        raw.insert(raw.end(), hb[ci].begin(), hb[ci].end());
     }
     if (have_prepared_ && std::memcmp(&prepared_, &knobs, sizeof(BatchKnobs)) == 0 && raw == prepared_boxes_raw_)
         return "";
@@ -150,6 +178,13 @@ std::string BatchEngine::prepare(const double *dt_scale) {
         Class &c = cls_[ci];
         const int nb = (int)c.boxes.size();
         const int V = knobs.plan[batch_size_index(c.N)] ? 1 : 0;
+        CUDA_TRY(cudaMemcpy(c.d_boxes, hb[ci].data(), hb[ci].size(), cudaMemcpyHostToDevice));
+        if (c.box) {
+            c.grid = c.group * nb;
+            c.step_items = 0;
+            for (int p = 0; p < kBoxPhases; ++p) c.step_items += (long long)c.items[p] * nb;
+            continue;
+        }
         std::string e = K_->setup(c.N, V, c.smem, &c.fit);
         if (!e.empty()) return e;
         if (c.fit < 1) return "batch: the batch kernel does not fit on an SM";
@@ -168,7 +203,6 @@ std::string BatchEngine::prepare(const double *dt_scale) {
                 }
         c.nsegs = (int)segs.size();
         c.step_items = first;
-        CUDA_TRY(cudaMemcpy(c.d_boxes, hb[ci].data(), sizeof(BatchBox) * nb, cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(c.d_segs, segs.data(), sizeof(BatchSeg) * segs.size(), cudaMemcpyHostToDevice));
     }
     for (auto &g : graphs_) cudaGraphExecDestroy(g.second);
@@ -188,7 +222,18 @@ std::string BatchEngine::capture_body(int nsteps) {
         const int V = knobs.plan[batch_size_index(c.N)] ? 1 : 0;
         CUDA_TRY(cudaEventRecord(c.fork, stream_));
         CUDA_TRY(cudaStreamWaitEvent(c.side, c.fork, 0));
-        if (knobs.mode == 0) {
+        if (c.box && knobs.mode == 0 && c.group) {
+            BoxLaunch l;
+            l.group = c.group;
+            l.boxes = nb;
+            l.cluster = true;
+            l.stream = c.side;
+            CUDA_TRY(box_kernels(precision_).run(c.N, V, l, BoxRun{}, (const BoxRun *)c.d_boxes, nsteps));
+        } else if (c.box) {
+            for (int s = 0; s < nsteps; ++s)
+                for (int p = 0; p < kBoxPhases; ++p)
+                    CUDA_TRY(K_->box_phase(c.N, V, p, nb, c.side, (const BoxRun *)c.d_boxes));
+        } else if (knobs.mode == 0) {
             CUDA_TRY(cudaMemsetAsync(c.d_ctr, 0, sizeof(unsigned long long) * (nb + 1), c.side));
             BatchArgs a{};
             a.boxes = (const BatchBox *)c.d_boxes;

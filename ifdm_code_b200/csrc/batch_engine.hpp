@@ -14,7 +14,8 @@ int batch_size_index(int n);     // -1 if n is not a batch size
 
 // Launch shape of the batch: the choices the autotuner makes.
 struct BatchKnobs {
-    int mode = 0;                 // 0: one persistent kernel per box size; 1: one launch per phase and size
+    int mode = 0;                 // 0: one kernel per box size for all steps where that is the faster; 1: one launch per phase and size
+    // tiled boxes only (128^3 in FP64 arithmetic; the others are one cluster of CTAs each):
     int blocks_per_sm = 2;        // persistent CTAs per SM (clamped to what fits)
     int group = 0;                // boxes per group in the persistent item order (0: all boxes in lock step)
     int plan[kBatchSizes] = {0};  // radix-plan variant per grid size
@@ -33,8 +34,8 @@ class BatchEngine {
     // which the batch orders itself against.
     std::string init(const std::vector<StepEngine *> &boxes, cudaStream_t stream);
     // nsteps fixed-mode steps of every box (dt_scale[b] per box), replayed
-    // from a captured CUDA graph: boxes of one size share one persistent
-    // launch (mode 0) or one launch per phase (mode 1); sizes run side by
+    // from a captured CUDA graph: boxes of one size share one launch (mode 0:
+    // a cluster of CTAs per box) or one launch per phase (mode 1); sizes run side by
     // side.  Asynchronous.
     std::string step(int nsteps, const double *dt_scale);
     // Time candidate knobs on trial_steps steps each (the boxes' states are
@@ -53,6 +54,8 @@ class BatchEngine {
         std::vector<int> boxes;         // indices into boxes_
         int items[10] = {0};            // items per phase of one box
         size_t smem = 0;
+        bool box = false;               // boxes whose plane fits a CTA: the one-launch kernels
+        int group = 0;                  // box: CTAs of the cluster that runs one box, 0: a launch per phase
         int fit = 0, grid = 0, nsegs = 0;
         long long step_items = 0;
         void *d_boxes = nullptr, *d_segs = nullptr;

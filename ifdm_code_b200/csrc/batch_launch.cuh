@@ -6,6 +6,7 @@
 #pragma once
 
 #include "batch_kernels.cuh"
+#include "box_launch.cuh"
 
 #include <string>
 
@@ -19,7 +20,11 @@ struct BatchKernels {
     cudaError_t (*persistent)(int N, int V, int grid, size_t smem, cudaStream_t s, const BatchArgs &a);
     cudaError_t (*phase)(int N, int V, int ph, int tiles, int nboxes, size_t smem, cudaStream_t s,
                          const BatchBox *boxes);
+    // the per-phase kernels of the boxes whose plane fits a CTA (box_kernels.cuh)
+    std::string (*box_setup)(int N, int V);
+    cudaError_t (*box_phase)(int N, int V, int ph, int nboxes, cudaStream_t s, const BoxRun *boxes);
 };
+constexpr int kBoxPhases = 6;  // timestep, A .. E
 
 const BatchKernels &batch_kernels(int precision);  // 0 FP64, 1 FP32, 2 mixed
 
@@ -62,34 +67,78 @@ template <typename R, typename K, int N, int V> struct BatchLaunch {
     }
 };
 
-// (N, V) -> BatchLaunch; V = 1 exists where PlanV<N, 1> differs from Plan<N>
-template <typename R, typename K, typename F> static bool with_batch_nv(int N, int V, F &&f) {
-    switch (N) {
-        case 16: f(BatchLaunch<R, K, 16, 0>{}); return true;
-        case 32: V ? f(BatchLaunch<R, K, 32, 1>{}) : f(BatchLaunch<R, K, 32, 0>{}); return true;
-        case 48: V ? f(BatchLaunch<R, K, 48, 1>{}) : f(BatchLaunch<R, K, 48, 0>{}); return true;
-        case 64: V ? f(BatchLaunch<R, K, 64, 1>{}) : f(BatchLaunch<R, K, 64, 0>{}); return true;
-        case 96: V ? f(BatchLaunch<R, K, 96, 1>{}) : f(BatchLaunch<R, K, 96, 0>{}); return true;
-        case 128: f(BatchLaunch<R, K, 128, 0>{}); return true;
-        default: return false;
+// Sizes whose plane does not fit a CTA (128 in FP64 arithmetic) run the tiles of the ten passes.
+template <typename R, typename K, typename F> static bool with_batch_nv(int N, int, F &&f) {
+    if constexpr (!box_fits<R, K, 128>()) {
+        if (N == 128) {
+            f(BatchLaunch<R, K, 128, 0>{});
+            return true;
+        }
     }
+    return false;
+}
+// f(BoxOps) of an (N, V) box that fits
+template <typename R, typename K, typename F> static bool with_box_nv(int N, int V, F &&f) {
+    if (V) {
+        switch (N) {
+            case 32: f(BoxOps<R, K, 32, 1>{}); return true;
+            case 48: f(BoxOps<R, K, 48, 1>{}); return true;
+            case 64: f(BoxOps<R, K, 64, 1>{}); return true;
+            case 96: f(BoxOps<R, K, 96, 1>{}); return true;
+            default: break;
+        }
+    }
+    return BoxTable<R, K>::with_n(N, f);
 }
 
 template <typename R, typename K> struct BatchTable {
-    template <int N> static void fill(int *items, size_t *smem) {
-        for (int p = 0; p < kBatchPhases; ++p) items[p] = batch_items<R, K, N>(p);
-        *smem = batch_smem<R, K, N>();
-    }
     static bool items(int N, int *it, size_t *smem) {
-        switch (N) {
-            case 16: fill<16>(it, smem); return true;
-            case 32: fill<32>(it, smem); return true;
-            case 48: fill<48>(it, smem); return true;
-            case 64: fill<64>(it, smem); return true;
-            case 96: fill<96>(it, smem); return true;
-            case 128: fill<128>(it, smem); return true;
-            default: return false;
+        for (int p = 0; p < kBatchPhases; ++p) it[p] = 0;
+        *smem = 0;
+        if (with_box_nv<R, K>(N, 0, [](auto) {})) {
+            for (int p = 0; p < kBoxPhases; ++p) it[p] = p ? N : 1;
+            return true;
         }
+        return with_batch_nv<R, K>(N, 0, [&](auto l) {
+            for (int p = 0; p < kBatchPhases; ++p) it[p] = batch_items<R, K, 128>(p);
+            *smem = batch_smem<R, K, 128>();
+        });
+    }
+    template <typename RR, typename KK, int N, int V> static std::string set_phases(BoxOps<RR, KK, N, V>) {
+        using O = BoxOps<RR, KK, N, V>;
+        const void *ph[kBoxPhases] = {(const void *)k_box_phase<RR, KK, N, V, 0>, (const void *)k_box_phase<RR, KK, N, V, 1>,
+                                      (const void *)k_box_phase<RR, KK, N, V, 2>, (const void *)k_box_phase<RR, KK, N, V, 3>,
+                                      (const void *)k_box_phase<RR, KK, N, V, 4>, (const void *)k_box_phase<RR, KK, N, V, 5>};
+        for (const void *f : ph) {
+            cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)O::SMEM);
+            if (e != cudaSuccess) return std::string("batch kernel setup: ") + cudaGetErrorString(e);
+        }
+        return "";
+    }
+    static std::string box_setup(int N, int V) {
+        std::string e = "batch: res " + std::to_string(N) + " has no plane kernels";
+        with_box_nv<R, K>(N, V, [&](auto o) { e = set_phases(o); });
+        return e;
+    }
+    template <typename RR, typename KK, int N, int V>
+    static cudaError_t one_phase(BoxOps<RR, KK, N, V>, int ph, int nb, cudaStream_t s, const BoxRun *b) {
+        using O = BoxOps<RR, KK, N, V>;
+        const dim3 g(ph ? unsigned(N) : 1u, unsigned(nb));
+        switch (ph) {
+            case 0: k_box_phase<RR, KK, N, V, 0><<<g, O::NT, O::SMEM, s>>>(b); break;
+            case 1: k_box_phase<RR, KK, N, V, 1><<<g, O::NT, O::SMEM, s>>>(b); break;
+            case 2: k_box_phase<RR, KK, N, V, 2><<<g, O::NT, O::SMEM, s>>>(b); break;
+            case 3: k_box_phase<RR, KK, N, V, 3><<<g, O::NT, O::SMEM, s>>>(b); break;
+            case 4: k_box_phase<RR, KK, N, V, 4><<<g, O::NT, O::SMEM, s>>>(b); break;
+            case 5: k_box_phase<RR, KK, N, V, 5><<<g, O::NT, O::SMEM, s>>>(b); break;
+            default: return cudaErrorInvalidValue;
+        }
+        return cudaGetLastError();
+    }
+    static cudaError_t box_phase(int N, int V, int ph, int nb, cudaStream_t s, const BoxRun *b) {
+        cudaError_t e = cudaErrorInvalidValue;
+        with_box_nv<R, K>(N, V, [&](auto o) { e = one_phase(o, ph, nb, s, b); });
+        return e;
     }
     static std::string setup(int N, int V, size_t smem, int *fit) {
         std::string e = "batch: res " + std::to_string(N) + " is not a batch size";
@@ -108,7 +157,7 @@ template <typename R, typename K> struct BatchTable {
         return e;
     }
     static const BatchKernels &table() {
-        static const BatchKernels t{&items, &setup, &persistent, &phase};
+        static const BatchKernels t{&items, &setup, &persistent, &phase, &box_setup, &box_phase};
         return t;
     }
 };

@@ -41,4 +41,16 @@ struct Phys {
     int limit;        // quadrature interval limit on the device
 };
 
+// Coefficients of one recorded step, as its passes used them.
+struct StepLog {
+    double coefP;        // kick coefficient of the stored phi
+    double coefQ;        // kick coefficient of |psi_s|^2
+    double alpha;        // dither phase of the kick
+    double drift_s;      // drift phase per unit kappa^2
+    double cre, cim;     // offset c of this step
+    double pendP, pendQ; // half kick owed after this step
+    double gphase;       // accumulated dither after this step's kick
+    double a, dt_KE, dt_PE, dt_QI;
+};
+
 }  // namespace ifdm

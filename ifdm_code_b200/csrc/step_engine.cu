@@ -7,6 +7,7 @@
 #include "zpass_pipe.cuh"
 #include "zpass_tma.cuh"
 #include "adjoint_kernels.cuh"
+#include "box_launch.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -16,6 +17,8 @@
 #include <cstring>
 #include <type_traits>
 #include <algorithm>
+#include <array>
+#include <map>
 #include <mutex>
 #include <set>
 
@@ -480,8 +483,16 @@ static std::string get_twiddles(int n, int prec, void **out) {
     return "";
 }
 
+const BoxKernels &box_kernels_fp64();
+const BoxKernels &box_kernels_fp32();
+const BoxKernels &box_kernels_mixed();
+const BoxKernels &box_kernels(int precision) {
+    return precision == 0 ? box_kernels_fp64() : precision == 1 ? box_kernels_fp32() : box_kernels_mixed();
+}
+
 // ------------------------------------------------------------ StepEngine --
 StepEngine::~StepEngine() {
+    cudaFree(box_scr_);
     cudaFree(psi_);
     cudaFree(phi_);
     cudaFree(rhok_);
@@ -563,12 +574,77 @@ std::string StepEngine::init(const EngineConfig &cfg, cudaStream_t stream) {
     const long tot = long(N) * N * N;
     win_rows_ = tot / P;
     win_tail_ = int(tot - win_rows_ * P);
+    return init_box();
+}
+
+// Whole runs in one launch where a plane of the box fits a CTA.
+// IFDM_NO_FUSE keeps the one-launch-per-pass kernels.
+std::string StepEngine::init_box() {
+    const int N = cfg_.N;
+    const BoxKernels &bk = box_kernels(cfg_.precision);
+    if (!bk.fits(N)) return "";
+    // one CTA per plane; a cluster where that is a cluster (its barrier takes
+    // 1000-2000 cycles against 3000 of the counter in global memory), else a cooperative grid
+    box_group_ = N;
+    box_cluster_ = N <= 16;
+    bool runs = false;
+    {
+        // attributes and the occupancy query once per device, size and precision
+        std::lock_guard<std::mutex> lk(setup_mutex());
+        static std::map<std::array<int, 3>, bool> known;
+        int dev = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        const std::array<int, 3> key{dev, N, cfg_.precision};
+        auto it = known.find(key);
+        if (it == known.end()) {
+            std::string e = bk.setup(N, 0);
+            if (!e.empty()) return e;
+            it = known.emplace(key, bk.resident(N, box_group_, box_cluster_) >= 1).first;
+        }
+        runs = it->second;
+    }
+    box_ = runs && std::getenv("IFDM_NO_FUSE") == nullptr;
+    CUDA_TRY(cudaMalloc(&box_scr_, sizeof(BoxScratch)));
+    CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
+    return "";
+}
+
+// timestep: 1 each step's own (appended to log when given), 0 the one *ts_
+// holds (one step), 2 replay log[0 ..] with step counters steps0 ...; save: keep
+// the state before each step in the segment buffers.
+std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void *log, long long steps0, bool save) {
+    BoxRun a{};
+    a.psi = psi_;
+    a.phi = phi_;
+    a.rhok = rhok_;
+    a.tw = tw_;
+    a.ts = ts_;
+    a.scr = (BoxScratch *)box_scr_;
+    a.ph = phys_;
+    a.ph.dt_scale = dt_scale;
+    a.win_rows = win_rows_;
+    a.win_tail = win_tail_;
+    a.timestep = timestep;
+    BoxLaunch l;
+    l.group = box_group_;
+    l.cluster = box_cluster_;
+    l.stream = stream_;
+    const size_t n3 = n3_(), rs = storage_bytes(cfg_.precision);
+    constexpr int kMaxSteps = 512;  // steps per launch (tens of milliseconds at 128^3)
+    for (int n = 0; n < nsteps; n += kMaxSteps) {
+        const int cnt = std::min(kMaxSteps, nsteps - n);
+        a.log = log ? (StepLog *)log + n : nullptr;
+        a.steps0 = steps0 + n;
+        a.seg_psi = save ? (char *)seg_psi_ + size_t(n) * n3 * 2 * rs : nullptr;
+        a.seg_phi = save ? (char *)seg_phi_ + size_t(n) * n3 * rs : nullptr;
+        CUDA_TRY(box_kernels(cfg_.precision).run(cfg_.N, 0, l, a, nullptr, cnt));
+    }
     return "";
 }
 
 size_t StepEngine::n3_() const { return size_t(cfg_.N) * cfg_.N * cfg_.N; }
 
-std::string StepEngine::set_physics(double a, double rhoc) {
+void StepEngine::set_physics(double rhoc) {
     using namespace phys;
     cfg_.rhoc = rhoc;
     const double m = cfg_.mfdm, ms = cfg_.mfdm_solar;
@@ -591,6 +667,9 @@ std::string StepEngine::set_physics(double a, double rhoc) {
     ph.N = cfg_.N;
     ph.dither = (cfg_.precision == 1 && std::getenv("IFDM_NO_DITHER") == nullptr) ? 1 : 0;
     ph.limit = 64;
+}
+
+std::string StepEngine::reset_state(double a) {
     TState t;
     std::memset(&t, 0, sizeof t);
     t.a = a;
@@ -600,12 +679,17 @@ std::string StepEngine::set_physics(double a, double rhoc) {
 }
 
 std::string StepEngine::load_psi(const double *psi, bool on_device, double a, double rhoc) {
-    std::string e = set_physics(a, rhoc);
-    if (!e.empty()) return e;
+    set_physics(rhoc);
     const size_t n3 = n3_();
     const double invS = 1.0 / S_;
     const int prec = cfg_.precision;
-    if (on_device) {
+    if (!box_) {
+        std::string e = reset_state(a);
+        if (!e.empty()) return e;
+    }
+    if (on_device && box_) {
+        // the initial pass reads psi itself
+    } else if (on_device) {
         if (prec == 0) k_psi_in<double><<<1184, 256, 0, stream_>>>((const double2 *)psi, (double2 *)psi_, invS, n3);
         else k_psi_in<float><<<1184, 256, 0, stream_>>>((const double2 *)psi, (float2 *)psi_, invS, n3);
 
@@ -634,6 +718,27 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         }
         // the caller may reuse its buffer once every copy has landed
         CUDA_TRY(cudaStreamSynchronize(copy_stream_));
+    }
+    if (box_) {
+        BoxRun a0{};
+        a0.psi = psi_;
+        a0.phi = phi_;
+        a0.rhok = rhok_;
+        a0.tw = tw_;
+        a0.ts = ts_;
+        a0.scr = (BoxScratch *)box_scr_;
+        a0.win_rows = win_rows_;
+        a0.win_tail = win_tail_;
+        a0.in = on_device ? psi : nullptr;
+        a0.invS = invS;
+        a0.a0 = a;
+        BoxLaunch l;
+        l.group = box_group_;
+        l.cluster = box_cluster_;
+        l.stream = stream_;
+        CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
+        CUDA_TRY(box_kernels(prec).load(cfg_.N, l, a0));
+        return "";
     }
     return launch_initial_density();
 }
@@ -687,7 +792,7 @@ std::string StepEngine::launch_initial_density() {
 std::string StepEngine::launch_timestep(double dt_scale) {
     Phys ph = phys_;
     ph.dt_scale = dt_scale;
-    const int nt = cfg_.N < 32 ? 32 : (cfg_.N > 512 ? 512 : cfg_.N);
+    const int nt = std::max(32, std::min(kTimestepThreads, cfg_.N));
     k_timestep<<<1, nt, 0, stream_>>>(ts_, ph, drift64_, drift32_);
     CUDA_TRY(cudaGetLastError());
     return "";
@@ -714,9 +819,13 @@ std::string StepEngine::launch_passes(cudaEvent_t *ev) {
 }
 
 std::string StepEngine::timestep_only(double dt_scale) { return launch_timestep(dt_scale); }
-std::string StepEngine::passes_only() { return launch_passes(nullptr); }
+std::string StepEngine::passes_only() {
+    if (box_) return box_run(1, 0, 1.0, nullptr, 0, false);
+    return launch_passes(nullptr);
+}
 
 std::string StepEngine::step(int nsteps, double dt_scale) {
+    if (box_) return box_run(nsteps, 1, dt_scale, nullptr, 0, false);
     for (int i = 0; i < nsteps; ++i) {
         std::string e = launch_timestep(dt_scale);
         if (!e.empty()) return e;
@@ -857,6 +966,13 @@ std::string StepEngine::record(int nsteps, double dt_scale, int ckpt) {
             CUDA_TRY(cudaMemcpyAsync((char *)ckpt_psi_ + k * n3 * cs, psi_, n3 * cs, cudaMemcpyDeviceToDevice, stream_));
             CUDA_TRY(cudaMemcpyAsync((char *)ckpt_phi_ + k * n3 * rs, phi_, n3 * rs, cudaMemcpyDeviceToDevice, stream_));
         }
+        if (box_) {  // up to the next checkpoint
+            const int cnt = std::min(ckpt - n % ckpt, nsteps - n);
+            e = box_run(cnt, 1, dt_scale, lg + n, 0, false);
+            if (!e.empty()) return e;
+            n += cnt - 1;
+            continue;
+        }
         e = launch_timestep(dt_scale);
         if (!e.empty()) return e;
         k_log_step<<<1, 1, 0, stream_>>>(ts_, lg + n);
@@ -924,6 +1040,11 @@ std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
     else
         k_scale_in<float><<<1184, 256, 0, stream_>>>((const double2 *)g_final_dev, (float2 *)g_, S_ * lambda, n3);
     CUDA_TRY(cudaGetLastError());
+    if (box_) {
+        std::string eb = adjoint_box(fin);
+        if (!eb.empty()) return eb;
+        return adjoint_finish(g0_dev, lambda);
+    }
     // the output map: psi_out = S psi exp(-i (pendP phi + pendQ |psi|^2 - gphase))
     std::string e = adjoint_kick(psi_, phi_, fin.pendP, fin.pendP, fin.pendQ, -fin.gphase, 1ll << 40);
     if (!e.empty()) return e;
@@ -970,7 +1091,12 @@ std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
             if (!e.empty()) return e;
         }
     }
-    // gradient with respect to the natural-unit psi_0 = S psi_s: g0 = g_s / S
+    return adjoint_finish(g0_dev, lambda);
+}
+
+// gradient with respect to the natural-unit psi_0 = S psi_s: g0 = g_s / S
+std::string StepEngine::adjoint_finish(double *g0_dev, double lambda) {
+    const size_t n3 = n3_();
     if (cfg_.precision == 0)
         k_scale_out<double><<<1184, 256, 0, stream_>>>((const double2 *)g_, (double2 *)g0_dev, 1.0 / S_, n3);
     else
@@ -978,6 +1104,54 @@ std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
                                                       n3);
     CUDA_TRY(cudaGetLastError());
     recorded_ = 0;  // the replay consumed the state; record again before another adjoint
+    return "";
+}
+
+// The sweep over the recorded steps with the one-launch kernels: per segment
+// the checkpoint's copy, one replay launch that keeps the states before its
+// steps, and one backward launch.  The last state of a segment stays in
+// psi_, phi_.
+std::string StepEngine::adjoint_box(const TState &fin) {
+    const size_t n3 = n3_();
+    const size_t rs = storage_bytes(cfg_.precision), cs = 2 * rs;
+    const int M = recorded_, K = ckpt_every_;
+    BoxSweep a{};
+    a.g = g_;
+    a.rhok = rhok_;
+    a.tw = tw_;
+    a.scr = (BoxScratch *)box_scr_;
+    a.err = &ts_->err;
+    a.log = (const StepLog *)log_;
+    a.seg_psi = seg_psi_;
+    a.seg_phi = seg_phi_;
+    a.last_psi = psi_;
+    a.last_phi = phi_;
+    BoxLaunch l;
+    l.group = box_group_;
+    l.cluster = box_cluster_;
+    l.stream = stream_;
+    const BoxKernels &bk = box_kernels(cfg_.precision);
+    // the output map: psi_out = S psi exp(-i (pendP phi + pendQ |psi|^2 - gphase))
+    a.start = a.end = M;
+    a.a = fin.pendP;
+    a.b = fin.pendQ;
+    a.alpha = -fin.gphase;
+    CUDA_TRY(bk.sweep(cfg_.N, l, a));
+    for (int seg = (M - 1) / K; seg >= 0; --seg) {
+        const int start = seg * K, end = std::min(M, start + K);
+        CUDA_TRY(cudaMemcpyAsync(psi_, (char *)ckpt_psi_ + size_t(seg) * n3 * cs, n3 * cs, cudaMemcpyDeviceToDevice,
+                                 stream_));
+        CUDA_TRY(cudaMemcpyAsync(phi_, (char *)ckpt_phi_ + size_t(seg) * n3 * rs, n3 * rs, cudaMemcpyDeviceToDevice,
+                                 stream_));
+        if (end - start > 1) {
+            // same step counters as the forward pass, so stochastic rounding repeats exactly
+            std::string e = box_run(end - start - 1, 2, 1.0, (StepLog *)log_ + start, start + 1, true);
+            if (!e.empty()) return e;
+        }
+        a.start = start;
+        a.end = end;
+        CUDA_TRY(bk.sweep(cfg_.N, l, a));
+    }
     return "";
 }
 

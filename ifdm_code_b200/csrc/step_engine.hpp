@@ -31,6 +31,7 @@ struct EngineView {
     Phys phys;  // dt_scale 1
     long win_rows;
     int win_tail;
+    void *box_scr;  // scratch of the one-launch kernels, null where a plane does not fit
 };
 
 // Names of the fused passes in launch order (timestep first).
@@ -85,14 +86,15 @@ class StepEngine {
     size_t n3() const { return size_t(cfg_.N) * cfg_.N * cfg_.N; }
     void *psi_ptr() const { return psi_; }
     EngineView view() const {
-        return {cfg_.N, cfg_.precision, psi_, phi_, rhok_, tw_, twh_, ts_, drift64_, drift32_, phys_, win_rows_, win_tail_};
+        return {cfg_.N, cfg_.precision, psi_, phi_, rhok_, tw_, twh_, ts_, drift64_, drift32_, phys_, win_rows_, win_tail_, box_scr_};
     }
 
   private:
     std::string launch_timestep(double dt_scale);
     std::string launch_passes(cudaEvent_t *ev);  // ev: optional 10 events (after each pass)
     std::string launch_initial_density();
-    std::string set_physics(double a, double rhoc);
+    void set_physics(double rhoc);
+    std::string reset_state(double a);
     std::string ensure_staging();
     size_t n3_() const;
 
@@ -120,6 +122,14 @@ class StepEngine {
     CUtensorMap map_psi_y_{}, map_psi_x_{}, map_rho_y_{}, map_rho_x_{};
     int tma_ly_ = 8, tma_lx_ = 8;  // lines per TMA tile of the y and x passes (inner box extent)
     // adjoint buffers
+    // one-launch box kernels (box_kernels.cuh): N <= 128 where a plane fits
+    bool box_ = false, box_cluster_ = false;
+    int box_group_ = 0;        // CTAs of the group that runs this box
+    void *box_scr_ = nullptr;  // BoxScratch
+    std::string init_box();
+    std::string box_run(int nsteps, int timestep, double dt_scale, void *log, long long steps0, bool save);
+    std::string adjoint_box(const TState &fin);
+    std::string adjoint_finish(double *g0_dev, double lambda);
     void *log_ = nullptr;  // StepLog[log_cap_]
     int log_cap_ = 0, recorded_ = 0, ckpt_every_ = 0, nckpt_cap_ = 0, seg_cap_ = 0;
     void *ckpt_psi_ = nullptr, *ckpt_phi_ = nullptr, *seg_psi_ = nullptr, *seg_phi_ = nullptr;

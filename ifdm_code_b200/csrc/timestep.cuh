@@ -1,13 +1,13 @@
 // timestep.cuh -- Timestep_criteria (src/CosmoBEC_MPI.cpp:19-78) on the device.
 //
-// One block.  Thread 0 turns the max reductions of the previous passes into
-// the three step criteria and advances the scale factor; three warps integrate
+// One warp turns the max reductions of the previous passes into the three
+// step criteria, advances the scale factor and integrates
 //   dt_KE = int da/(H a^3), dt_PE = int da/(H a^2), dt_QI = int da/(H a^4)
 // (integrands src/struct3D.h:127-146) with the QUADPACK method the reference
 // gets from GSL's qags: one 21-point Gauss-Kronrod rule, accepted when its
 // error estimate meets epsrel = 1e-10, else bisection of the worst interval.
-// It then writes the merged kick coefficients for the next z-pass and all
-// threads fill the separable drift tables exp(-i s kappa_i^2).
+// It writes the merged kick coefficients for the next kick; the block's
+// threads then fill the separable drift tables exp(-i s kappa_i^2).
 #pragma once
 
 #include "step_kernels.cuh"
@@ -202,90 +202,182 @@ static __global__ void k_reduce_init(TState *__restrict__ ts, const double *__re
     }
 }
 
-// The timestep.  drift64/drift32: tables exp(-i s kappa_i^2), i < N.  Run by
-// one block: thread 0 does the scalar work, all threads fill the tables.
-__device__ __forceinline__ void timestep_body(TState *ts, const Phys &ph, double2 *drift64, float2 *drift32) {
-    __shared__ double s_drift, s_ai, s_da, s_int[3];
-    __shared__ int s_bad[3];
-    if (threadIdx.x == 0) {
-        const double maxphi = ph.Phi0 * bits_to_double(ts->maxphi_bits);
-        const double maxrho = ph.S2 * bits_to_double(ts->maxrho_bits);
-        ts->maxphi_bits = 0ull;
-        ts->maxrho_bits = 0ull;
-        ts->maxphi = maxphi;
-        ts->maxrho = maxrho;
-        const double ai = ts->a;
-        const double dt_KE = ph.A_KE * (ai * ai);
-        const double dt_PE = ph.B_PE / maxphi * ai;
-        double dt_QI = ph.C_QI / maxrho * (ai * ai * ai);
-        if (ph.g == 0) dt_QI = 0.0;
-        double max_dt = dt_KE;
-        int crit = 3;
-        if (max_dt > dt_PE) { max_dt = dt_PE; crit = 2; }
-        if ((max_dt > dt_QI) && (ph.g != 0)) { max_dt = dt_QI; crit = 4; }
-        max_dt *= ph.dt_scale;
-        const double H = ph.H0 * sqrt(ph.Om / (ai * ai * ai) + (1.0 - ph.Om));
-        const double da = H * ai * max_dt;
-        s_ai = ai;
-        s_da = da;
-        ts->cand_KE = dt_KE;
-        ts->cand_PE = dt_PE;
-        ts->cand_QI = dt_QI;
-        ts->da = da;
-        ts->crit = crit;
+// Append the current step to a log.
+__device__ __forceinline__ void log_step(const TState *ts, StepLog *lg) {
+    StepLog e;
+    e.coefP = ts->coefP;
+    e.coefQ = ts->coefQ;
+    e.alpha = ts->alpha;
+    e.drift_s = ts->drift_s;
+    e.cre = ts->cre;
+    e.cim = ts->cim;
+    e.pendP = ts->pendP;
+    e.pendQ = ts->pendQ;
+    e.gphase = ts->gphase;
+    e.a = ts->a;
+    e.dt_KE = ts->dt_KE;
+    e.dt_PE = ts->dt_PE;
+    e.dt_QI = ts->dt_QI;
+    *lg = e;
+}
+
+// The 21-point rule laid out by lane (0-9 left nodes, 10-19 right, 20 centre,
+// the rest zero): signed abscissa, Kronrod weight, Gauss weight.
+struct GkNodes {
+    double x[32], wk[32], wg[32];
+};
+__device__ __forceinline__ void gk_fill(GkNodes *g) {  // threads 0..31; the caller syncs
+    const int i = threadIdx.x;
+    if (i >= 32) return;
+    const int j = i < 20 ? i % 10 : 10;
+    g->x[i] = i < 10 ? -c_gk_x[j] : (i < 20 ? c_gk_x[j] : 0.0);
+    g->wk[i] = i < 21 ? c_gk_wk[j] : 0.0;
+    g->wg[i] = i < 20 && j % 2 ? c_gk_wg[j / 2] : 0.0;
+}
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The timestep, by one full warp, in two parts: the kinetic criterion depends
+// on a alone, so the integrals over a kinetic-limited step can be computed
+// before the reductions of the previous step are complete (the one-launch
+// kernels do it while they wait for them) and are used when that criterion
+// limits the step.  One warp takes the three integrals together: each lane evaluates its
+// node's H once, the powers a^2, a^3, a^4 by multiplication and the three
+// quotients side by side, and the sums run over the warp in parallel (the
+// same rule, sums in another order; an interval whose error estimate misses
+// 1e-10 goes to the bisecting qags_dev).  Latency is all that counts here, one
+// warp's dependent FP64 chain: with pow() per node, the integrals on three
+// warps and sequential 21-term sums the kernel took 12-14 us of every step.
+struct StepIntegrals {
+    double dt;       // the criterion's step before the scale
+    double da, r[3]; // int da/(H a^n) over [a, a + da], n = 3, 2, 4
+    int bad;
+};
+static __device__ __noinline__ int qags_warp(int n, double H0, double Om, double a, double b, int limit, double *r) {
+    return qags_dev<true>(n, H0, Om, a, b, limit, r);
+}
+__device__ __forceinline__ double kinetic_dt(double ai, const Phys &ph) { return ph.A_KE * (ai * ai); }
+static __device__ __noinline__ void step_integrals(double ai, double max_dt, const Phys &ph, const GkNodes *gk,
+                                                   StepIntegrals *out) {
+    const int lane = threadIdx.x & 31;
+    const double H = ph.H0 * sqrt(ph.Om / (ai * ai * ai) + (1.0 - ph.Om));
+    const double da = H * ai * (max_dt * ph.dt_scale);
+    const double lo = ai, hi = ai + da, c = 0.5 * (lo + hi), h = 0.5 * (hi - lo);
+    const double x = c + h * gk->x[lane], wk = gk->wk[lane], wg = gk->wg[lane];
+    const double x2 = x * x, x3 = x2 * x, Hx = ph.H0 * sqrt(ph.Om / x3 + (1.0 - ph.Om));
+    const double f[3] = {1.0 / (Hx * x3), 1.0 / (Hx * x2), 1.0 / (Hx * (x2 * x2))};
+    double kron[3], gauss[3], sasc[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        kron[q] = warp_sum(wk * f[q]);
+        gauss[q] = warp_sum(wg * f[q]);
     }
-    __syncthreads();
-    // the three integrals of a to a + da, one full warp each (with fewer full
-    // warps they take them in turn; a partial last warp stays out, its
-    // shuffles need all 32 lanes); each warp evaluates a 21-point rule in one go
-    const int wid = (int)(threadIdx.x >> 5), nfull = (int)(blockDim.x >> 5);
-    for (int q = wid; wid < nfull && q < 3; q += nfull) {
-        double r;
-        const int bad = qags_dev<true>(q == 0 ? 3 : (q == 1 ? 2 : 4), ph.H0, ph.Om, s_ai, s_ai + s_da, ph.limit, &r);
-        if ((threadIdx.x & 31) == 0) {
-            s_int[q] = r;
-            s_bad[q] = bad;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) sasc[q] = warp_sum(wk * fabs(f[q] - 0.5 * kron[q])) * fabs(h);
+    int bad = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        double err = fabs((kron[q] - gauss[q]) * h), r = kron[q] * h;
+        if (sasc[q] != 0.0 && err != 0.0) {
+            const double e = 200.0 * err / sasc[q], scale = e * sqrt(e);
+            err = scale < 1.0 ? sasc[q] * scale : sasc[q];
         }
+        err = fmax(err, 50.0 * 2.220446049250313e-16 * fabs(r));  // the integrands are positive
+        if (!((err <= 1e-10 * fabs(r) && err != sasc[q]) || err == 0.0))
+            bad |= qags_warp(q == 0 ? 3 : (q == 1 ? 2 : 4), ph.H0, ph.Om, lo, hi, ph.limit, &r);
+        if (lane == 0) out->r[q] = r;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double ai = s_ai, da = s_da;
-        const double iKE = s_int[0], iPE = s_int[1], iQI = s_int[2];
-        if (s_bad[0] | s_bad[1] | s_bad[2]) ts->err |= 1;
-        ts->dt_KE = iKE;
-        ts->dt_PE = iPE;
-        ts->dt_QI = iQI;
-        ts->a = ai + da;
-        const double hp = 0.5 * iPE * ph.kP, hq = 0.5 * iQI * ph.kQ;
-        ts->snapP = ts->pendP;
-        ts->snapQ = ts->pendQ;
-        ts->coefP = ts->pendP + hp;
-        ts->coefQ = ts->pendQ + hq;
-        ts->pendP = hp;
-        ts->pendQ = hq;
-        ts->drift_s = ph.kin * iKE;
-        // global-phase dither (FP32 mode): psi is stored as exp(-i gphase) psi
-        // and this step's kick adds alpha, a pseudo-random phase in [0, 2 pi)
-        // from the step count, so consecutive steps round different numbers;
-        // the offset c (a mean of psi) rotates with it
-        double alpha = 0.0;
-        if (ph.dither) {
-            const unsigned long long h = (unsigned long long)ts->steps * 0x9e3779b97f4a7c15ull + 0x632be59bd9b4e019ull;
-            const unsigned long long m = (h ^ (h >> 31)) * 0xbf58476d1ce4e5b9ull;
-            alpha = 6.283185307179586476925286766559 * (double)((m ^ (m >> 29)) >> 11) * 0x1.0p-53;
-        }
-        double sa, ca;
+    if (lane == 0) {
+        out->dt = max_dt;
+        out->da = da;
+        out->bad = bad;
+    }
+    __syncwarp();
+}
+
+// *ts and *si in shared memory, *si the integrals of the kinetic step of
+// ts->a; the reductions and the mean of the kicked field (cn_re, cn_im) come
+// from the previous step.  Written by lane 0; the caller syncs.
+static __device__ __noinline__ void timestep_warp(TState *ts, const Phys &ph, const GkNodes *gk, StepIntegrals *si,
+                                                  unsigned long long phi_bits, unsigned long long rho_bits, double cn_re,
+                                                  double cn_im) {
+    const double maxphi = ph.Phi0 * bits_to_double(phi_bits);
+    const double maxrho = ph.S2 * bits_to_double(rho_bits);
+    const double ai = ts->a;
+    const double dt_KE = si->dt;
+    const double dt_PE = ph.B_PE / maxphi * ai;
+    double dt_QI = ph.C_QI / maxrho * (ai * ai * ai);
+    if (ph.g == 0) dt_QI = 0.0;
+    double max_dt = dt_KE;
+    int crit = 3;
+    if (max_dt > dt_PE) { max_dt = dt_PE; crit = 2; }
+    if ((max_dt > dt_QI) && (ph.g != 0)) { max_dt = dt_QI; crit = 4; }
+    if (crit != 3) step_integrals(ai, max_dt, ph, gk, si);
+    if ((threadIdx.x & 31) != 0) return;
+    if (si->bad) ts->err |= 1;
+    ts->maxphi = maxphi;
+    ts->maxrho = maxrho;
+    ts->cand_KE = dt_KE;
+    ts->cand_PE = dt_PE;
+    ts->cand_QI = dt_QI;
+    ts->da = si->da;
+    ts->crit = crit;
+    const double iKE = si->r[0], iPE = si->r[1], iQI = si->r[2];
+    ts->dt_KE = iKE;
+    ts->dt_PE = iPE;
+    ts->dt_QI = iQI;
+    ts->a = ai + si->da;
+    const double hp = 0.5 * iPE * ph.kP, hq = 0.5 * iQI * ph.kQ;
+    const double pp = ts->pendP, pq = ts->pendQ;
+    ts->snapP = pp;
+    ts->snapQ = pq;
+    ts->coefP = pp + hp;
+    ts->coefQ = pq + hq;
+    ts->pendP = hp;
+    ts->pendQ = hq;
+    ts->drift_s = ph.kin * iKE;
+    // global-phase dither (FP32 mode): psi is stored as exp(-i gphase) psi
+    // and this step's kick adds alpha, a pseudo-random phase in [0, 2 pi)
+    // from the step count, so consecutive steps round different numbers;
+    // the offset c (a mean of psi) rotates with it
+    double alpha = 0.0, sa = 0.0, ca = 1.0;
+    if (ph.dither) {
+        const unsigned long long k = (unsigned long long)ts->steps * 0x9e3779b97f4a7c15ull + 0x632be59bd9b4e019ull;
+        const unsigned long long m = (k ^ (k >> 31)) * 0xbf58476d1ce4e5b9ull;
+        alpha = 6.283185307179586476925286766559 * (double)((m ^ (m >> 29)) >> 11) * 0x1.0p-53;
         sincos(alpha, &sa, &ca);
-        ts->alpha = alpha;
-        ts->gphase_prev = ts->gphase;
-        ts->gphase = fmod(ts->gphase + alpha, 6.283185307179586476925286766559);
-        ts->cre = ts->cnext_re * ca + ts->cnext_im * sa;
-        ts->cim = ts->cnext_im * ca - ts->cnext_re * sa;
-        ts->steps += 1;
-        s_drift = ph.kin * iKE;
+    }
+    const double g0 = ts->gphase, gp = g0 + alpha, twopi = 6.283185307179586476925286766559;
+    ts->alpha = alpha;
+    ts->gphase_prev = g0;
+    ts->gphase = gp >= twopi ? gp - twopi : gp;  // both in [0, 2 pi): the subtraction is exact
+    ts->cre = cn_re * ca + cn_im * sa;
+    ts->cim = cn_im * ca - cn_re * sa;
+    ts->steps += 1;
+}
+
+// The timestep of *ts (global memory) by one block; all threads fill the
+// tables exp(-i s kappa_i^2), i < N.
+__device__ __forceinline__ void timestep_body(TState *ts, const Phys &ph, double2 *drift64, float2 *drift32) {
+    __shared__ TState st;
+    __shared__ GkNodes gk;
+    __shared__ StepIntegrals si;
+    gk_fill(&gk);
+    if (threadIdx.x == 0) st = *ts;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        step_integrals(st.a, kinetic_dt(st.a, ph), ph, &gk, &si);
+        timestep_warp(&st, ph, &gk, &si, st.maxphi_bits, st.maxrho_bits, st.cnext_re, st.cnext_im);
+        if (threadIdx.x == 0) {
+            st.maxphi_bits = st.maxrho_bits = 0ull;
+            *ts = st;
+        }
     }
     __syncthreads();
-    const double s = s_drift;
+    const double s = st.drift_s;
     const double twopi = 6.283185307179586476925286766559;
     for (int i = threadIdx.x; i < ph.N; i += blockDim.x) {
         const double k = (double)kappa(i, ph.N);
@@ -298,7 +390,8 @@ __device__ __forceinline__ void timestep_body(TState *ts, const Phys &ph, double
     }
 }
 
-static __global__ void k_timestep(TState *__restrict__ ts, Phys ph, double2 *__restrict__ drift64,
+constexpr int kTimestepThreads = 256;
+static __global__ void __launch_bounds__(kTimestepThreads) k_timestep(TState *__restrict__ ts, Phys ph, double2 *__restrict__ drift64,
                            float2 *__restrict__ drift32) {
     timestep_body(ts, ph, drift64, drift32);
 }
