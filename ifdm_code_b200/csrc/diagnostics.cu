@@ -1,4 +1,4 @@
-// diagnostics.cu -- power spectrum of the density contrast on the device.
+// diagnostics.cu -- power spectrum and energy means of a box on the device.
 //
 // P(k) of delta = rho / <rho> - 1, rho = |psi|^2, estimated on the full FFT
 // grid: P(k_b) = <|delta_k|^2>_b L^3 / N^6 averaged over the modes of
@@ -6,17 +6,24 @@
 // k = 2 pi kappa / L).  The reference has no such output; it is the measure
 // the precision comparisons of the step use, so it runs where psi lives.
 //
-//   1. rho into a complex128 work array (imaginary part 0) and its sum
-//      (fixed-order block sums);
-//   2. the 3-D c2c FFT of this project (fft3d);
-//   3. one block per group of 16 (x, y) lines: for every bin present in a
-//      line, a fixed-order block reduction of |rho_k|^2, |kappa| and the mode
-//      count; thread 0 adds the line sums in line order -> per-group partials;
-//   4. one block per bin adds the group partials in order.
-// Every sum has a fixed order, so the result does not change between runs.
+//   1. z pass: rho from psi as it is stored (a kick does not change it), its
+//      sum, the real-to-half FFT along z in FP64;
+//   2. FFTs along y and x of the half spectrum;
+//   3. the bins: a warp takes whole (x, y) lines in a fixed order; the modes of a
+//      bin within 32 consecutive kz are added by a warp tree, the bin's sums in
+//      line order (kz between 0 and N/2 stands for -kz too);
+//   4. one block per bin adds the partial sums in order.
+// 66 bytes a cell (FP64 psi); a full complex transform of rho after writing psi
+// out took 184.  Every sum has a fixed order, so the result does not change between runs.
+//
+// Energy means: the gradient's mean by Parseval, one axis at a time: sum over k of kappa_z^2
+// |psi_k|^2 is N^2 times the sum over the lines along z of their own
+// transforms, so three one-axis transforms that write nothing replace the
+// three-dimensional one (72 bytes a cell instead of 176).
 #include "diagnostics.hpp"
-#include "step_engine.hpp"
+#include "step_kernels.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -30,12 +37,16 @@ namespace ifdm {
 
 namespace {
 
-constexpr int kSumBlocks = 592, kSumThreads = 256;  // 4 blocks per SM
-constexpr int kLinesPerBlock = 16, kBinThreads = 128;
+constexpr int kBinBlocks = 592, kBinThreads = 256;  // 4 blocks per SM
+constexpr int kBinWarps = kBinThreads / 32;
 
-__device__ __forceinline__ double block_sum(double v, double *red) {
+__device__ __forceinline__ double wsum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ double block_sum(double v, double *red) {
+    v = wsum(v);
     const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[w] = v;
@@ -45,111 +56,161 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
     return t;
 }
 
-// rho = |psi|^2 (in place: psi -> (rho, 0)); part[block] = sum over the block's elements
-__global__ void k_rho_sum(double2 *__restrict__ d, size_t n, double *__restrict__ part) {
-    __shared__ double red[32];
+// FP64 row tiles whatever psi's storage type R
+template <int N> using DTile = TileZ<double, double, N>;
+
+// rho = |psi_s|^2, part[block] its sum, real-to-half FFT along z -> rk [row][NHP]
+template <typename R, int N>
+__global__ void __launch_bounds__(DTile<N>::NT)
+    k_rho_half_z(const cx<R> *__restrict__ psi, double2 *__restrict__ rk, double *__restrict__ part,
+                 const double2 *__restrict__ tw, const double2 *__restrict__ twh) {
+    using TL = DTile<N>;
+    constexpr int NH = N / 2 + 1, NHP = half_pitch<double>(N), M = N / 2, PER = TL::L * N / TL::NT;
+    static_assert(PER * TL::NT == TL::L * N, "whole rows per thread block");
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double2 *sm = reinterpret_cast<double2 *>(smraw);
+    double *smr = reinterpret_cast<double *>(smraw);
+    const size_t row0 = size_t(blockIdx.x) * TL::L, base = row0 * N;
+    cx<R> g[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) g[i] = psi[base + threadIdx.x + i * TL::NT];
     double s = 0.0;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const double2 v = d[i];
-        const double r = v.x * v.x + v.y * v.y;
-        d[i] = make_double2(r, 0.0);
-        s += r;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int f = threadIdx.x + i * TL::NT, l = f / N, n = f % N;
+        const double n2 = cnorm2(cin<double>(g[i]));
+        s += n2;
+        smr[2 * ((n >> 1) * TL::LP + l) + (n & 1)] = n2;
     }
-    const double t = block_sum(s, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    __shared__ double out[3];
+    block_sum3(s, 0.0, 0.0, out);  // syncs
+    if (threadIdx.x == 0) part[blockIdx.x] = out[0];
+    fft_tile<double2, M, TL::EH, -1, TL::L, TL::LP, typename TL::HP>(sm, twh);
+    constexpr int TPR = TL::NT / TL::L;  // threads per row
+    const int l = threadIdx.x / TPR;
+    for (int k = threadIdx.x % TPR; k < NH; k += TPR) {
+        const double2 zk = sm[(k % M) * TL::LP + l];
+        const double2 zc = cconj(sm[((M - k) % M) * TL::LP + l]);
+        const double2 e = cscale(zk + zc, 0.5);
+        const double2 wo = post_tw<-1, N>(tw, k % N, cscale(zk - zc, 0.5));
+        rk[(row0 + l) * NHP + k] = mkc(e.x + wo.y, e.y - wo.x);
+    }
 }
 
-__global__ void k_sum_parts(const double *__restrict__ part, int n, double *__restrict__ out) {
+// psi with the pending half kick (as ifdm_get_psi, in storage units) -> out;
+// part[5 block ..]: sums of |psi|^2, |psi|^4, phi |psi|^2, kappa_z^2 |FFT_z|^2
+template <typename R, int N>
+__global__ void __launch_bounds__(DTile<N>::NT)
+    k_energy_z(const cx<R> *__restrict__ psi, const R *__restrict__ phi, const TState *__restrict__ ts,
+               double2 *__restrict__ out, double *__restrict__ part, const double2 *__restrict__ tw) {
+    using TL = DTile<N>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double2 *sm = reinterpret_cast<double2 *>(smraw);
+    const size_t base = size_t(blockIdx.x) * TL::L * N;
+    const double cp = ts->pendP, cq = ts->pendQ, g = ts->gphase;
+    double a = 0.0, b = 0.0, c = 0.0, k2 = 0.0;
+    for (int f = threadIdx.x; f < TL::L * N; f += TL::NT) {
+        const double2 v = cin<double>(psi[base + f]);
+        const double p = (double)phi[base + f], r = cnorm2(v);
+        double sn, cs;
+        sincos(cp * p + cq * r - g, &sn, &cs);
+        const double2 w = mkc(v.x * cs + v.y * sn, v.y * cs - v.x * sn);
+        out[base + f] = w;
+        sm[(f % N) * TL::LP + f / N] = w;
+        a += r;
+        b += r * r;
+        c += p * r;
+    }
+    __syncthreads();
+    fft_tile<double2, N, TL::E, -1, TL::L, TL::LP>(sm, tw);
+    for (int f = threadIdx.x; f < TL::L * N; f += TL::NT) {
+        const double k = (double)kappa(f % N, N);
+        k2 = fma(k * k, cnorm2(sm[(f % N) * TL::LP + f / N]), k2);
+    }
+    __shared__ double o[6];
+    block_sum3(a, b, c, o);
+    __syncthreads();  // the second sum reuses block_sum3's words
+    block_sum3(k2, 0.0, 0.0, o + 3);
+    if (threadIdx.x == 0)
+        for (int i = 0; i < 4; ++i) part[5 * size_t(blockIdx.x) + i] = o[i];
+}
+
+// out[c] = sum over blocks b (in order) of part[stride b + c], c < nv
+__global__ void k_sum_cols(const double *__restrict__ part, int nb, int stride, int nv, double *__restrict__ out) {
     __shared__ double red[32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
-    const double t = block_sum(s, red);
-    if (threadIdx.x == 0) *out = t;
+    for (int c = 0; c < nv; ++c) {
+        double a = 0.0;
+        for (int b = threadIdx.x; b < nb; b += blockDim.x) a += part[size_t(stride) * b + c];
+        a = block_sum(a, red);
+        if (threadIdx.x == 0) out[c] = a;
+    }
 }
 
 struct BinEdges {
     double e[kMaxBins + 1];
 };
 
-__device__ __forceinline__ int bin_of(double kk, const BinEdges &ed, int nb) {
-    if (!(kk >= ed.e[0]) || !(kk < ed.e[nb])) return -1;
-    int lo = 0, hi = nb;  // ed.e[lo] <= kk < ed.e[hi]
+__device__ __forceinline__ int bin_of(double kk, const double *e, int nb) {
+    if (!(kk >= e[0]) || !(kk < e[nb])) return -1;
+    int lo = 0, hi = nb;  // e[lo] <= kk < e[hi]
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (kk >= ed.e[mid]) lo = mid;
+        if (kk >= e[mid]) lo = mid;
         else hi = mid;
     }
     return lo;
 }
 
-// part[(group * nb + b) * 3 + {0,1,2}] = sum |rho_k|^2, sum |kappa|, modes
-template <int PER>
+// part[(block * nb + b) * 3 + {0,1,2}] = sum |rho_k|^2, sum |kappa|, modes
 __global__ void __launch_bounds__(kBinThreads)
-    k_bin_lines(const double2 *__restrict__ rk, int N, int nb, BinEdges ed, double *__restrict__ part) {
-    __shared__ double red[32];
-    __shared__ double acc[3 * kMaxBins];
-    __shared__ int brange[2];
-    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) acc[i] = 0.0;
-    const size_t lines = size_t(N) * N;
-    for (int q = 0; q < kLinesPerBlock; ++q) {
-        const size_t line = size_t(blockIdx.x) * kLinesPerBlock + q;
-        if (line >= lines) break;
+    k_bin_half(const double2 *__restrict__ rk, int N, int pitch, int nb, BinEdges ed, double *__restrict__ part) {
+    __shared__ double e[kMaxBins + 1];
+    __shared__ double acc[kBinWarps][3 * kMaxBins];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i <= nb; i += blockDim.x) e[i] = ed.e[i];
+    for (int i = lane; i < 3 * nb; i += 32) acc[w][i] = 0.0;
+    __syncthreads();
+    const int M = N / 2;
+    const long lines = long(N) * N;
+    for (long line = long(blockIdx.x) * kBinWarps + w; line < lines; line += long(gridDim.x) * kBinWarps) {
         const int ix = int(line / N), iy = int(line % N);
-        const double kx = ix < N / 2 ? ix : ix - N, ky = iy < N / 2 ? iy : iy - N;
-        double p[PER], kk[PER];
-        int b[PER];
-        int bmin = kMaxBins, bmax = -1;
-#pragma unroll
-        for (int e = 0; e < PER; ++e) {
-            const int iz = threadIdx.x + e * kBinThreads;
-            b[e] = -1;
-            p[e] = 0.0;
-            kk[e] = 0.0;
-            if (iz < N) {
-                const double kz = iz < N / 2 ? iz : iz - N;
-                kk[e] = sqrt(kx * kx + ky * ky + kz * kz);
-                b[e] = bin_of(kk[e], ed, nb);
-                const double2 v = rk[line * N + iz];
-                p[e] = kk[e] > 0.0 ? v.x * v.x + v.y * v.y : 0.0;  // delta_0 = 0
-                if (b[e] >= 0) {
-                    bmin = min(bmin, b[e]);
-                    bmax = max(bmax, b[e]);
+        const double kx = ix < M ? ix : ix - N, ky = iy < M ? iy : iy - N;
+        const double2 *row = rk + line * pitch;
+        for (int k0 = 0; k0 <= M; k0 += 32) {
+            const int iz = k0 + lane;
+            int b = -1, m = 0;
+            double p = 0.0, kk = 0.0;
+            if (iz <= M) {
+                const double kz = iz < M ? iz : iz - N;
+                m = iz == 0 || iz == M ? 1 : 2;
+                kk = sqrt(kx * kx + ky * ky + kz * kz);
+                b = bin_of(kk, e, nb);
+                const double2 v = row[iz];
+                p = kk > 0.0 ? m * (v.x * v.x + v.y * v.y) : 0.0;  // delta_0 = 0
+                kk *= m;
+            }
+            const int b1 = __reduce_max_sync(0xffffffffu, b);
+            if (b1 < 0) continue;
+            const int b0 = __reduce_min_sync(0xffffffffu, b < 0 ? kMaxBins : b);
+            for (int bb = b0; bb <= b1; ++bb) {
+                const bool in = b == bb;
+                const int cnt = __reduce_add_sync(0xffffffffu, in ? m : 0);
+                if (cnt == 0) continue;
+                const double sp = wsum(in ? p : 0.0), sk = wsum(in ? kk : 0.0);
+                if (lane == 0) {
+                    acc[w][3 * bb] += sp;
+                    acc[w][3 * bb + 1] += sk;
+                    acc[w][3 * bb + 2] += (double)cnt;
                 }
             }
         }
-        if (threadIdx.x == 0) {
-            brange[0] = kMaxBins;
-            brange[1] = -1;
-        }
-        __syncthreads();
-        if (bmax >= 0) {
-            atomicMin(&brange[0], bmin);
-            atomicMax(&brange[1], bmax);
-        }
-        __syncthreads();
-        const int b0 = brange[0], b1 = brange[1];
-        for (int bb = b0; bb <= b1; ++bb) {
-            double sp = 0.0, sk = 0.0, sc = 0.0;
-#pragma unroll
-            for (int e = 0; e < PER; ++e)
-                if (b[e] == bb) {
-                    sp += p[e];
-                    sk += kk[e];
-                    sc += 1.0;
-                }
-            sp = block_sum(sp, red);
-            sk = block_sum(sk, red);
-            sc = block_sum(sc, red);
-            if (threadIdx.x == 0) {
-                acc[3 * bb] += sp;
-                acc[3 * bb + 1] += sk;
-                acc[3 * bb + 2] += sc;
-            }
-        }
-        __syncthreads();
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) part[size_t(blockIdx.x) * 3 * nb + i] = acc[i];
+    for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) {
+        double s = 0.0;
+        for (int q = 0; q < kBinWarps; ++q) s += acc[q][i];
+        part[size_t(blockIdx.x) * 3 * nb + i] = s;
+    }
 }
 
 // out[b * 3 + c] = sum over groups of part[(group * nb + b) * 3 + c]
@@ -164,97 +225,81 @@ __global__ void k_bin_total(const double *__restrict__ part, int groups, int nb,
     }
 }
 
-template <int PER>
-void launch_bins(const double2 *rk, int N, int nb, const BinEdges &ed, double *part, int groups, cudaStream_t s) {
-    k_bin_lines<PER><<<groups, kBinThreads, 0, s>>>(rk, N, nb, ed, part);
-}
-
-// sums over x of |psi|^2, |psi|^4 and phi |psi|^2: part[3 * block + {0, 1, 2}]
-__global__ void k_xsums(const double2 *__restrict__ psi, const double *__restrict__ phi, size_t n,
-                        double *__restrict__ part) {
-    __shared__ double red[32];
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const double2 v = psi[i];
-        const double r = v.x * v.x + v.y * v.y;
-        a += r;
-        b += r * r;
-        c += phi[i] * r;
-    }
-    a = block_sum(a, red);
-    b = block_sum(b, red);
-    c = block_sum(c, red);
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = a;
-        part[3 * blockIdx.x + 1] = b;
-        part[3 * blockIdx.x + 2] = c;
+template <typename F> std::string with_n(int n, F &&f) {
+    switch (n) {
+        case 16: return f(std::integral_constant<int, 16>{});
+        case 32: return f(std::integral_constant<int, 32>{});
+        case 48: return f(std::integral_constant<int, 48>{});
+        case 64: return f(std::integral_constant<int, 64>{});
+        case 96: return f(std::integral_constant<int, 96>{});
+        case 128: return f(std::integral_constant<int, 128>{});
+        case 256: return f(std::integral_constant<int, 256>{});
+        case 512: return f(std::integral_constant<int, 512>{});
+        case 1024: return f(std::integral_constant<int, 1024>{});
+        default: return "unsupported grid";
     }
 }
 
-// sum over k of |kappa|^2 |psi_k|^2 (kappa per axis in -N/2 .. N/2-1): part[block]
-__global__ void k_ksum(const double2 *__restrict__ pk, int N, double *__restrict__ part) {
-    __shared__ double red[32];
-    const size_t n3 = size_t(N) * N * N;
-    double a = 0.0;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n3; i += size_t(gridDim.x) * blockDim.x) {
-        const int ix = int(i / (size_t(N) * N)), iy = int((i / N) % N), iz = int(i % N);
-        const double kx = ix < N / 2 ? ix : ix - N, ky = iy < N / 2 ? iy : iy - N, kz = iz < N / 2 ? iz : iz - N;
-        const double2 v = pk[i];
-        a += (kx * kx + ky * ky + kz * kz) * (v.x * v.x + v.y * v.y);
-    }
-    a = block_sum(a, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
+// shared-memory attribute set at each call (cheap, and per device)
+template <typename Kern> cudaError_t big_smem(Kern k, size_t bytes) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// out[c] = sum over blocks b (in order) of part[nv * b + c], c < nv
-__global__ void k_sum_cols(const double *__restrict__ part, int nb, int nv, double *__restrict__ out) {
-    __shared__ double red[32];
-    for (int c = 0; c < nv; ++c) {
-        double a = 0.0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) a += part[size_t(nv) * b + c];
-        a = block_sum(a, red);
-        if (threadIdx.x == 0) out[c] = a;
-    }
-}
+// workspace: [0, 5 N^2/8) z partial sums, [.., + N^2) axis partial sums, bin parts, totals
+size_t off_axis(int N) { return size_t(5) * N * N / 8; }
+size_t off_bins(int N) { return off_axis(N) + size_t(N) * N; }
+size_t off_out(int N) { return off_bins(N) + size_t(kBinBlocks) * 3 * kMaxBins; }
 
 }  // namespace
 
-std::string field_means(double2 *psi_work, const double *phi, int N, double xmax, double out[4], cudaStream_t s) {
-    if (N < 2 || N > 1024) return "unsupported grid";
-    const size_t n3 = size_t(N) * N * N;
-    double *d_part = nullptr;
-    std::string err;
-    auto run = [&]() -> std::string {
-        DG_TRY(cudaMalloc(&d_part, sizeof(double) * (4 * kSumBlocks + 4)));
-        double *d_tot = d_part + 4 * kSumBlocks;
-        k_xsums<<<kSumBlocks, kSumThreads, 0, s>>>(psi_work, phi, n3, d_part);
-        k_sum_cols<<<1, 1024, 0, s>>>(d_part, kSumBlocks, 3, d_tot);
-        DG_TRY(cudaGetLastError());
-        const std::string e = fft3d(psi_work, N, 0, -1, s);
-        if (!e.empty()) return e;
-        k_ksum<<<kSumBlocks, kSumThreads, 0, s>>>(psi_work, N, d_part + 3 * kSumBlocks);
-        k_sum_cols<<<1, 1024, 0, s>>>(d_part + 3 * kSumBlocks, kSumBlocks, 1, d_tot + 3);
-        DG_TRY(cudaGetLastError());
-        double h[4];
-        DG_TRY(cudaMemcpyAsync(h, d_tot, sizeof(h), cudaMemcpyDeviceToHost, s));
-        DG_TRY(cudaStreamSynchronize(s));
-        const double inv = 1.0 / double(n3), kf = 3.14159265358979323846 / xmax;  // k = pi kappa / xmax
-        out[0] = h[0] * inv;
-        out[1] = h[3] * inv * inv * kf * kf;  // Parseval: sum_x |grad psi|^2 = sum_k k^2 |psi_k|^2 / N^3
-        out[2] = h[2] * inv;
-        out[3] = h[1] * inv;
-        return "";
-    };
-    err = run();
-    cudaFree(d_part);
-    return err;
+size_t diag_work_doubles(int N) { return off_out(N) + 3 * kMaxBins + 8; }
+
+std::string field_means(const EngineView &v, double S, double2 *field, double *work, double xmax, double out[4],
+                        cudaStream_t s) {
+    const int N = v.N;
+    const double n3 = double(N) * N * N;
+    double *tot = work + off_out(N);
+    const void *tw = nullptr, *twh = nullptr;
+    std::string e = twiddle_tables(N, 0, &tw, &twh);
+    if (!e.empty()) return e;
+    e = with_n(N, [&](auto n) -> std::string {
+        using TL = DTile<decltype(n)::value>;
+        static_assert(TL::L >= 8, "partial sums");
+        const int blocks = N * N / TL::L;
+        auto go = [&](auto kern, const auto *psi, const auto *phi) -> std::string {
+            DG_TRY(big_smem(kern, TL::SMEM));
+            kern<<<blocks, TL::NT, TL::SMEM, s>>>(psi, phi, v.ts, field, work, (const double2 *)tw);
+            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 5, 4, tot);
+            DG_TRY(cudaGetLastError());
+            return "";
+        };
+        if (v.precision == 0) return go(k_energy_z<double, decltype(n)::value>, (const double2 *)v.psi, (const double *)v.phi);
+        return go(k_energy_z<float, decltype(n)::value>, (const float2 *)v.psi, (const float *)v.phi);
+    });
+    for (int axis = 1; e.empty() && axis >= 0; --axis) {
+        int np = 0;
+        e = axis_k2(field, N, axis, work + off_axis(N), &np, s);
+        if (e.empty()) k_sum_cols<<<1, 1024, 0, s>>>(work + off_axis(N), np, 1, 1, tot + 4 + axis);
+    }
+    if (!e.empty()) return e;
+    double h[6];
+    DG_TRY(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, s));
+    DG_TRY(cudaStreamSynchronize(s));
+    const double S2 = S * S, kf = 3.14159265358979323846 / xmax;  // k = pi kappa / xmax
+    out[0] = h[0] / n3 * S2;
+    // Parseval per axis: sum_x |d psi/dz|^2 = sum over lines of sum_k k^2 |.|^2 / N
+    out[1] = (h[3] + h[4] + h[5]) / N / n3 * kf * kf * S2;
+    out[2] = h[2] / n3 * S2;
+    out[3] = h[1] / n3 * S2 * S2;
+    return "";
 }
 
-std::string power_spectrum(double2 *work, int N, double L, int nbins, const double *edges, double *k_out,
-                           double *pk_out, long long *modes_out, double *mean_rho, cudaStream_t s) {
+std::string power_spectrum(const EngineView &v, double S, double2 *field, double *work, double L, int nbins,
+                           const double *edges, double *k_out, double *pk_out, long long *modes_out, double *mean_rho,
+                           cudaStream_t s) {
+    const int N = v.N;
     if (nbins < 1 || nbins > kMaxBins) return "nbins must be 1.." + std::to_string(kMaxBins);
-    if (N < 2 || N > 1024) return "unsupported grid";
-    const size_t n3 = size_t(N) * N * N;
+    const double n3 = double(N) * N * N;
     BinEdges ed{};
     if (edges) {
         for (int i = 0; i <= nbins; ++i) {
@@ -268,45 +313,44 @@ std::string power_spectrum(double2 *work, int N, double L, int nbins, const doub
         ed.e[0] = 1.0;
         ed.e[nbins] = N / 2.0;
     }
-    const int groups = int((size_t(N) * N + kLinesPerBlock - 1) / kLinesPerBlock);
-    double *d_part = nullptr, *d_out = nullptr;
-    std::string err;
-    auto run = [&]() -> std::string {
-        DG_TRY(cudaMalloc(&d_part, sizeof(double) * std::max<size_t>(kSumBlocks, size_t(groups) * 3 * nbins)));
-        DG_TRY(cudaMalloc(&d_out, sizeof(double) * (3 * kMaxBins + 1)));
-        k_rho_sum<<<kSumBlocks, kSumThreads, 0, s>>>(work, n3, d_part);
-        k_sum_parts<<<1, 1024, 0, s>>>(d_part, kSumBlocks, d_out + 3 * kMaxBins);
-        DG_TRY(cudaGetLastError());
-        const std::string e = fft3d(work, N, 0, -1, s);
-        if (!e.empty()) return e;
-        const int per = (N + kBinThreads - 1) / kBinThreads;
-        if (per <= 1) launch_bins<1>(work, N, nbins, ed, d_part, groups, s);
-        else if (per <= 2) launch_bins<2>(work, N, nbins, ed, d_part, groups, s);
-        else if (per <= 4) launch_bins<4>(work, N, nbins, ed, d_part, groups, s);
-        else launch_bins<8>(work, N, nbins, ed, d_part, groups, s);
-        DG_TRY(cudaGetLastError());
-        k_bin_total<<<nbins, 256, 0, s>>>(d_part, groups, nbins, d_out);
-        DG_TRY(cudaGetLastError());
-        std::vector<double> h(3 * kMaxBins + 1);
-        DG_TRY(cudaMemcpyAsync(h.data(), d_out, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
-        DG_TRY(cudaStreamSynchronize(s));
-        const double sum = h[3 * kMaxBins], mean = sum / double(n3);
-        if (mean_rho) *mean_rho = mean;
-        // delta_k = rho_k / mean for kappa != 0 (the bins exclude kappa = 0)
-        const double twopi = 6.283185307179586476925286766559;
-        const double norm = (L * L * L) / (double(n3) * double(n3)) / (mean * mean);
-        for (int b = 0; b < nbins; ++b) {
-            const double cnt = h[3 * b + 2];
-            if (modes_out) modes_out[b] = (long long)cnt;
-            if (pk_out) pk_out[b] = cnt > 0 ? h[3 * b] / cnt * norm : 0.0;
-            if (k_out) k_out[b] = cnt > 0 ? h[3 * b + 1] / cnt * twopi / L : 0.0;
-        }
-        return "";
-    };
-    err = run();
-    cudaFree(d_part);
-    cudaFree(d_out);
-    return err;
+    double *tot = work + off_out(N);
+    const void *tw = nullptr, *twh = nullptr;
+    std::string e = twiddle_tables(N, 0, &tw, &twh);
+    if (!e.empty()) return e;
+    e = with_n(N, [&](auto n) -> std::string {
+        using TL = DTile<decltype(n)::value>;
+        const int blocks = N * N / TL::L;
+        auto go = [&](auto kern, const auto *psi) -> std::string {
+            DG_TRY(big_smem(kern, TL::SMEM));
+            kern<<<blocks, TL::NT, TL::SMEM, s>>>(psi, field, work, (const double2 *)tw, (const double2 *)twh);
+            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 1, 1, tot + 3 * kMaxBins);
+            DG_TRY(cudaGetLastError());
+            return "";
+        };
+        if (v.precision == 0) return go(k_rho_half_z<double, decltype(n)::value>, (const double2 *)v.psi);
+        return go(k_rho_half_z<float, decltype(n)::value>, (const float2 *)v.psi);
+    });
+    if (e.empty()) e = fft_half_axis(field, N, 1, s);
+    if (e.empty()) e = fft_half_axis(field, N, 0, s);
+    if (!e.empty()) return e;
+    k_bin_half<<<kBinBlocks, kBinThreads, 0, s>>>(field, N, half_pitch<double>(N), nbins, ed, work + off_bins(N));
+    k_bin_total<<<nbins, 256, 0, s>>>(work + off_bins(N), kBinBlocks, nbins, tot);
+    DG_TRY(cudaGetLastError());
+    std::vector<double> h(3 * kMaxBins + 1);
+    DG_TRY(cudaMemcpyAsync(h.data(), tot, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
+    DG_TRY(cudaStreamSynchronize(s));
+    const double mean = h[3 * kMaxBins] / n3;
+    if (mean_rho) *mean_rho = mean * S * S;
+    // delta_k = rho_k / mean for kappa != 0 (the bins exclude kappa = 0)
+    const double twopi = 6.283185307179586476925286766559;
+    const double norm = (L * L * L) / (n3 * n3) / (mean * mean);
+    for (int b = 0; b < nbins; ++b) {
+        const double cnt = h[3 * b + 2];
+        if (modes_out) modes_out[b] = (long long)cnt;
+        if (pk_out) pk_out[b] = cnt > 0 ? h[3 * b] / cnt * norm : 0.0;
+        if (k_out) k_out[b] = cnt > 0 ? h[3 * b + 1] / cnt * twopi / L : 0.0;
+    }
+    return "";
 }
 
 }  // namespace ifdm

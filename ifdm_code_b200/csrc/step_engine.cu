@@ -54,6 +54,11 @@ bool supported_n(int n, int precision) {
     return supported_n(n);
 }
 
+// map of one axis pass over a caller's field: axis 1 [planes][N][N], axis 0 [N][planes][N]; L lines a tile
+static std::string make_field_map(CUtensorMap *m, void *base, bool f64, int N, int planes, int axis, int L);
+static std::string make_axis_maps(CUtensorMap *my, CUtensorMap *mx, void *base, bool f64, int N, int W, int Ly,
+                                  int Lx, int boxr);
+
 // ---------------------------------------------------------------- per-N ops --
 template <typename R_, typename K_, int N> struct Box {
     using R = R_;
@@ -100,6 +105,10 @@ template <typename R_, typename K_, int N> struct Box {
         CUDA_TRY(prep(k_fft_z<R, K, N, +1>, SMZ));
         CUDA_TRY(prep(k_source_r2c_z<R, K, N>, SMZ));
         CUDA_TRY(prep(k_fft_x_poisson_slab<R, K, N>, SM));
+        if constexpr (std::is_same<R, double>::value && N < 256) {
+            CUDA_TRY(prep(k_line_k2<N, 1>, SM));
+            CUDA_TRY(prep(k_line_k2<N, 2>, SM));
+        }
         int sms = 0;
         CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         if constexpr (kZPipe) {
@@ -121,7 +130,11 @@ template <typename R_, typename K_, int N> struct Box {
             zt1grid = sms * (b1 > 0 ? b1 : 1);
             zt5grid = sms * (b5 > 0 ? b5 : 1);
             zt9grid = sms * (b9 > 0 ? b9 : 1);
+            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, -1>, ZSM5));
+            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, +1>, ZSM5));
             if constexpr (kPairZ) {
+                CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, -1>, ZSM5P));
+                CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, +1>, ZSM5P));
                 CUDA_TRY(prep(k_kick_fft_z_pair<N, ZST1P, ZB1P>, ZSM1P));
                 CUDA_TRY(prep(k_density_r2c_z_pair<N, ZST5P, ZB5P>, ZSM5P));
                 CUDA_TRY(prep(k_c2r_z_pair<N, ZST9P, ZB9P>, ZSM9P));
@@ -142,6 +155,14 @@ template <typename R_, typename K_, int N> struct Box {
             CUDA_TRY(prep(k_yx_tma<R, K, N, 1, 0, +1>, TT::SMEM));
             CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 1, 0>, TX::SMEM));
             CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 2, 0>, TX::SMEM));
+            if constexpr (kFftTma) {
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, -1>, TX::SMEM));
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, +1>, TX::SMEM));
+                if constexpr (std::is_same<R, double>::value) {
+                    CUDA_TRY(prep(k_line_k2_tma<N, 1>, TT::SMEM));
+                    CUDA_TRY(prep(k_line_k2_tma<N, 2>, TX::SMEM));
+                }
+            }
             // persistent grids: every block resident at once (one wave)
             int by = 0, bx = 0;
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by, k_yx_tma<R, K, N, 1, 0, -1>, TT::NT, TT::SMEM));
@@ -153,6 +174,8 @@ template <typename R_, typename K_, int N> struct Box {
                 CUDA_TRY(prep(k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY>, TPY::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 1, 0, PSTX, PBX>, TPX::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 2, 0, PSTX, PBX>, TPX::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, -1, PSTX, PBX>, TPX::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, +1, PSTX, PBX>, TPX::SMEM));
                 int py = 0, px = 0;
                 CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&py, k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY>,
                                                                        TPY::NT, TPY::SMEM));
@@ -171,6 +194,7 @@ template <typename R_, typename K_, int N> struct Box {
     // but slowed the FP64 z passes (one 2-slot block per SM hides less latency
     // than three plain blocks), and pipelined P1/P9 gained nothing.
     static constexpr bool kTma = N >= 128;
+    static constexpr bool kFftTma = N >= 256;  // the callers' own fields (axis_pass)
     static constexpr bool kZPipe = N >= 128 && N <= 512 && std::is_same<R, float>::value && std::is_same<K, float>::value;
     // z passes fed by bulk copies (zpass_tma.cuh) for N >= 256, FP32 and
     // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
@@ -337,6 +361,44 @@ template <typename R_, typename K_, int N> struct Box {
     // x-slab [planes][N][N], axis 1 = y on the x-slab, axis 0 = x on the
     // transposed y-slab [N][planes][N] (op 1: forward, -1/(kappa^2 N^3) with
     // global y offset y0, inverse).
+    // Forward pass along axis 1 (y) or 0 (x) of a half spectrum [N][N][NHP] (diagnostics; FP64)
+    static std::string half_axis(G *data, int axis, const C *tw, cudaStream_t s) {
+        if constexpr (kFftTma && std::is_same<R, double>::value) {
+            CUtensorMap my, mx;
+            std::string e = make_axis_maps(&my, &mx, data, true, N, NHP, TT::L, TX::L, N < 256 ? N : 256);
+            if (!e.empty()) return e;
+            if (axis == 1)
+                k_yx_tma<R, K, N, 1, 0, -1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, data, NHP, NH, int(size_t(N) * NHP / TT::L), nullptr, 6, nullptr, tw);
+            else
+                k_yx_tma<R, K, N, 2, 0, -1><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, data, NHP, NH, int(size_t(N) * NHP / TX::L), nullptr, 7, nullptr, tw);
+        } else if (axis == 1) {
+            k_fft_yx<R, K, N, -1, 1><<<hblocks(), TL::NT, SM, s>>>(data, NHP, NH, nullptr, 0, tw);
+        } else {
+            k_fft_yx<R, K, N, -1, 2><<<hblocks(), TL::NT, SM, s>>>(data, NHP, NH, nullptr, 0, tw);
+        }
+        return "";
+    }
+    // sum of kappa^2 |.|^2 over the forward transforms along axis 1 or 0 of a
+    // field [N][N][N] (diagnostics; FP64): one partial sum a block, *nparts of them
+    static std::string line_k2(const G *data, int axis, double *part, int *nparts, const C *tw, cudaStream_t s) {
+        if constexpr (std::is_same<R, double>::value) {
+            if constexpr (kFftTma) {
+                CUtensorMap my, mx;
+                std::string e = make_axis_maps(&my, &mx, const_cast<G *>(data), true, N, N, TT::L, TX::L, N < 256 ? N : 256);
+                if (!e.empty()) return e;
+                const int nt = int(size_t(N) * N / (axis == 1 ? TT::L : TX::L));
+                *nparts = axis == 1 ? ygrid : xgrid;
+                if (axis == 1) k_line_k2_tma<N, 1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, nt, tw, part);
+                else k_line_k2_tma<N, 2><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, nt, tw, part);
+            } else {
+                *nparts = int(zblocks());
+                if (axis == 1) k_line_k2<N, 1><<<zblocks(), TL::NT, SM, s>>>(data, tw, part);
+                else k_line_k2<N, 2><<<zblocks(), TL::NT, SM, s>>>(data, tw, part);
+            }
+            return "";
+        }
+        return "line_k2 needs FP64";
+    }
     static std::string fft_slab(G *data, int planes, int axis, int sign, int op, int y0, const C *tw, cudaStream_t s) {
         const size_t nl = size_t(planes) * N;
         if (nl % TL::L || nl % TZ::L) return "planes * n must be a multiple of the tile lines";
@@ -356,17 +418,53 @@ template <typename R_, typename K_, int N> struct Box {
         return "";
     }
 
-    static void fft3d(G *data, int sign, const C *tw, cudaStream_t s) {
-        const unsigned nt = TL::NT;
-        if (sign < 0) {
-            k_fft_z<R, K, N, -1><<<zrows(), TZ::NT, SMZ, s>>>(data, tw, 0x2545f491u);
-            k_fft_yx<R, K, N, -1, 1><<<zblocks(), nt, SM, s>>>(data, N, N, nullptr, 0, tw);
-            k_fft_yx<R, K, N, -1, 2><<<zblocks(), nt, SM, s>>>(data, N, N, nullptr, 0, tw);
-        } else {
-            k_fft_z<R, K, N, +1><<<zrows(), TZ::NT, SMZ, s>>>(data, tw, 0x2545f491u);
-            k_fft_yx<R, K, N, +1, 1><<<zblocks(), nt, SM, s>>>(data, N, N, nullptr, 0, tw);
-            k_fft_yx<R, K, N, +1, 2><<<zblocks(), nt, SM, s>>>(data, N, N, nullptr, 0, tw);
+    // One axis (2 = z, 1 = y, 0 = x) of the callers' field of planes * N lines
+    // (see fft_slab for the layouts) with the pipelined kernels of the steps;
+    // base 16-byte aligned (bulk copies), N >= 256.  One axis pass of 256^3
+    // complex128 measured 172 us plain.  Below 256 the field is in L2 and the
+    // passes are as long as their launches either way.
+    static std::string axis_pass(G *data, int planes, int axis, int sign, const C *tw, cudaStream_t s) {
+        if constexpr (kFftTma) {
+            const size_t lines = size_t(planes) * N;
+            if (axis == 2) {
+                if constexpr (kZT) {
+                    using Z = ZT<N, R>;
+                    const int nz = int(lines / Z::L);
+                    if constexpr (kPairZ) {
+                        if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
+                        else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
+                    } else {
+                        if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
+                        else k_fft_z_tma<N, ZST5, ZB5, R, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
+                    }
+                    return "";
+                }
+                return fft_slab(data, planes, axis, sign, 0, 0, tw, s);
+            }
+            CUtensorMap m;
+            std::string e = make_field_map(&m, data, std::is_same<R, double>::value, N, planes, axis, axis == 1 ? TT::L : TX::L);
+            if (!e.empty()) return e;
+            if constexpr (kPair) {
+                const int nt = int(lines / TPY::L);
+                if (axis == 1) {
+                    if (sign < 0) k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
+                    else k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
+                } else {
+                    if (sign < 0) k_yx_tma_pair<N, 2, 0, -1, PSTX, PBX><<<pxgrid, TPX::NT, TPX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                    else k_yx_tma_pair<N, 2, 0, +1, PSTX, PBX><<<pxgrid, TPX::NT, TPX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                }
+            } else if (axis == 1) {
+                const int nt = int(lines / TT::L);
+                if (sign < 0) k_yx_tma<R, K, N, 1, 0, -1><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
+                else k_yx_tma<R, K, N, 1, 0, +1><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
+            } else {
+                const int nt = int(lines / TX::L);
+                if (sign < 0) k_yx_tma<R, K, N, 2, 0, -1><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
+                else k_yx_tma<R, K, N, 2, 0, +1><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
+            }
+            return "";
         }
+        return fft_slab(data, planes, axis, sign, 0, 0, tw, s);
     }
 };
 
@@ -432,6 +530,21 @@ static std::string make_axis_maps(CUtensorMap *my, CUtensorMap *mx, void *base, 
     const cuuint64_t sx[1] = {cuuint64_t(2) * W * N * es};
     const cuuint32_t bx[2] = {cuuint32_t(2 * Lx), cuuint32_t(boxr)};
     return encode_map(mx, base, f64, 2, dx, sx, bx);
+}
+
+static std::string make_field_map(CUtensorMap *m, void *base, bool f64, int N, int planes, int axis, int L) {
+    const cuuint64_t es = f64 ? 8 : 4;
+    const cuuint32_t boxr = cuuint32_t(N < 256 ? N : 256);
+    if (axis == 1) {
+        const cuuint64_t d[3] = {cuuint64_t(2) * N, cuuint64_t(N), cuuint64_t(planes)};
+        const cuuint64_t st[2] = {cuuint64_t(2) * N * es, cuuint64_t(2) * N * N * es};
+        const cuuint32_t b[3] = {cuuint32_t(2 * L), boxr, 1};
+        return encode_map(m, base, f64, 3, d, st, b);
+    }
+    const cuuint64_t d[2] = {cuuint64_t(2) * N * planes, cuuint64_t(N)};
+    const cuuint64_t st[1] = {cuuint64_t(2) * N * planes * es};
+    const cuuint32_t b[2] = {cuuint32_t(2 * L), boxr};
+    return encode_map(m, base, f64, 2, d, st, b);
 }
 
 // arithmetic type of a precision mode: 0 double, 1 float
@@ -1155,6 +1268,9 @@ std::string StepEngine::adjoint_box(const TState &fin) {
     return "";
 }
 
+// bulk copies need a 16-byte base; a complex64 view may start at 8
+static bool field_aligned(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 std::string fft_slab(void *data, int n, int planes, int axis, int precision, int sign, int op, int y0,
                      cudaStream_t stream) {
     if (!supported_n(n, precision)) return "unsupported grid size " + std::to_string(n);
@@ -1167,11 +1283,49 @@ std::string fft_slab(void *data, int n, int planes, int axis, int precision, int
         using G = typename B::G;
         std::string e2 = B::configure();
         if (!e2.empty()) return e2;
-        e2 = B::fft_slab((G *)data, planes, axis, sign, op, y0, (const C *)tw, stream);
+        if (op == 0 && field_aligned(data) && planes * n % 16 == 0)
+            e2 = B::axis_pass((G *)data, planes, axis, sign, (const C *)tw, stream);
+        else e2 = B::fft_slab((G *)data, planes, axis, sign, op, y0, (const C *)tw, stream);
         if (!e2.empty()) return e2;
         CUDA_TRY(cudaGetLastError());
         return "";
     });
+}
+
+// FP64 pieces of the diagnostics: the N-point table, a half-spectrum axis
+// pass, the kappa^2 sums along an axis (Box::half_axis, Box::line_k2)
+template <typename F> static std::string with_fp64(int n, F &&f) {
+    if (!supported_n(n)) return "unsupported grid size " + std::to_string(n);
+    void *tw = nullptr;
+    std::string e = get_twiddles(n, 0, &tw);
+    if (!e.empty()) return e;
+    return with_box<double, double>(n, [&](auto box) -> std::string {
+        using B = decltype(box);
+        std::string e2 = B::configure();
+        if (!e2.empty()) return e2;
+        e2 = f(box, (const double2 *)tw);
+        if (!e2.empty()) return e2;
+        CUDA_TRY(cudaGetLastError());
+        return "";
+    });
+}
+std::string fft_half_axis(void *data, int n, int axis, cudaStream_t stream) {
+    return with_fp64(n, [&](auto box, const double2 *tw) {
+        return decltype(box)::half_axis((double2 *)data, axis, tw, stream);
+    });
+}
+std::string axis_k2(const void *data, int n, int axis, double *part, int *nparts, cudaStream_t stream) {
+    return with_fp64(n, [&](auto box, const double2 *tw) {
+        return decltype(box)::line_k2((const double2 *)data, axis, part, nparts, tw, stream);
+    });
+}
+std::string twiddle_tables(int n, int precision, const void **tw, const void **twh) {
+    void *a = nullptr, *b = nullptr;
+    std::string e = get_twiddles(n, compute_kind(precision), &a);
+    if (e.empty()) e = get_twiddles(n / 2, compute_kind(precision), &b);
+    *tw = a;
+    *twh = b;
+    return e;
 }
 
 std::string fft3d(void *data, int n, int precision, int sign, cudaStream_t stream) {
@@ -1185,7 +1339,11 @@ std::string fft3d(void *data, int n, int precision, int sign, cudaStream_t strea
         using G = typename B::G;
         std::string e2 = B::configure();
         if (!e2.empty()) return e2;
-        B::fft3d((G *)data, sign, (const C *)tw, stream);
+        for (int axis = 2; axis >= 0; --axis) {  // z, y, x
+            e2 = field_aligned(data) ? B::axis_pass((G *)data, n, axis, sign, (const C *)tw, stream)
+                                     : B::fft_slab((G *)data, n, axis, sign, 0, 0, (const C *)tw, stream);
+            if (!e2.empty()) return e2;
+        }
         CUDA_TRY(cudaGetLastError());
         return "";
     });

@@ -202,6 +202,112 @@ __global__ void __launch_bounds__(TmaTile<R, K, N, AXIS>::NT, TmaTile<R, K, N, A
     }
 }
 
+// Sum over all lines of kappa^2 |v_kappa|^2 of their forward transforms, one
+// axis of an FP64 field [N][N][N] that is only read: part[block] (fixed
+// order: a thread's elements, a warp tree, the warps).  The tiles and the
+// ring of k_yx_tma; bound by the one read (16 bytes a cell).
+template <int N, int AXIS>
+__global__ void __launch_bounds__(TmaTile<double, double, N, AXIS>::NT, TmaTile<double, double, N, AXIS>::MINB)
+    k_line_k2_tma(const __grid_constant__ CUtensorMap map, int ntiles, const double2 *__restrict__ tw,
+                  double *__restrict__ part) {
+    using TL = TmaTile<double, double, N, AXIS>;
+    using C = double2;
+    constexpr int L = TL::L, T = TL::T, ST = TL::STAGES, E = TL::E;
+    constexpr int R0 = Plan<N>::R[0], RL = Plan<N>::R[Plan<N>::NST - 1];
+    extern __shared__ __align__(128) unsigned char smraw[];
+    C *bufs = reinterpret_cast<C *>(smraw);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * TL::TILE_BYTES);
+    const int tid = threadIdx.x, l = tid % L, t = tid / L;
+    if (tid == 0) {
+        for (int s = 0; s < ST; ++s) mbar_init(&bar[s], 1);
+        mbar_init_fence();
+        prefetch_tmap(&map);
+    }
+    C *stw = reinterpret_cast<C *>(smraw + TL::TWOFF);
+    stage_twiddles(stw, tw, N);
+    const SmemTw<C> tws{stw};
+    __syncthreads();
+    const int my_n = blockIdx.x < (unsigned)ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    auto issue = [&](int i) {
+        const long g0 = ((long)blockIdx.x + (long)i * gridDim.x) * L;
+        const int s = i % ST;
+        C *dst = bufs + (size_t)s * N * L;
+        mbar_arrive_expect_tx(&bar[s], (uint32_t)TL::TILE_BYTES);
+#pragma unroll
+        for (int h = 0; h < N; h += TL::BOXR) {
+            if (AXIS == 1) tma_load_3d(dst + (size_t)h * L, &map, 2 * int(g0 % N), h, int(g0 / N), &bar[s]);
+            else tma_load_2d(dst + (size_t)h * L, &map, 2 * int(g0), h, &bar[s]);
+        }
+    };
+    if (tid == 0)
+        for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
+    double sum = 0.0;
+    for (int i = 0; i < my_n; ++i) {
+        const int s = i % ST;
+        if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
+        const bool ok = mbar_wait(&bar[s], (uint32_t)((i / ST) & 1), nullptr, 2);
+        if (!__syncthreads_and(ok)) {
+            // a load never completed: wait (bounded) for the copies still in flight, leave a NaN
+            if (tid == 0) {
+                for (int j = i; j < my_n && j <= i + ST - 1; ++j)
+                    mbar_wait(&bar[j % ST], (uint32_t)((j / ST) & 1), nullptr, 2);
+                part[blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
+            }
+            __syncthreads();
+            return;
+        }
+        C v[E];
+        C *wk = bufs + (size_t)s * N * L;
+        stage_load<C, N, E, L, L, R0>(wk, v, l, t);
+        stage_compute<C, N, E, -1, R0, 1>(v, tws, t);
+        RegChain<C, N, E, -1, L, L, 1, R0, TL::SWZ>::run(wk, v, tws, l, t, true);
+#pragma unroll
+        for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+            for (int r = 0; r < RL; ++r) {
+                const double k = (double)kappa(t + T * b + r * (N / RL), N);
+                sum = fma(k * k, cnorm2(v[b * RL + r]), sum);
+            }
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
+    // the block's sum in the ring (every copy has landed and been read): static
+    // shared memory would move the ring off the 128 bytes its copies need
+    double *red = reinterpret_cast<double *>(smraw);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) red[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        double tot = 0.0;
+        for (int i = 0; i < TL::NT / 32; ++i) tot += red[i];
+        part[blockIdx.x] = tot;
+    }
+}
+
+// The same sum from plain tiles (one a block), the sizes without a ring.
+template <int N, int AXIS>
+__global__ void __launch_bounds__(Tile<double, double, N>::NT)
+    k_line_k2(const double2 *__restrict__ data, const double2 *__restrict__ tw, double *__restrict__ part) {
+    using TL = Tile<double, double, N>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    double2 *sm = reinterpret_cast<double2 *>(smraw);
+    const int l = threadIdx.x % TL::L;
+    const long g = long(blockIdx.x) * TL::L + l;
+    const size_t b = line_base<AXIS>(g, N, N), S = AXIS == 1 ? size_t(N) : size_t(N) * N;
+    for (int n = threadIdx.x / TL::L; n < N; n += TL::NT / TL::L) sm[n * TL::LP + l] = data[b + n * S];
+    __syncthreads();
+    fft_tile<double2, N, TL::E, -1, TL::L, TL::LP>(sm, tw);
+    double sum = 0.0;
+    for (int n = threadIdx.x / TL::L; n < N; n += TL::NT / TL::L) {
+        const double k = (double)kappa(n, N);
+        sum = fma(k * k, cnorm2(sm[n * TL::LP + l]), sum);
+    }
+    __shared__ double out[3];
+    block_sum3(sum, 0.0, 0.0, out);
+    if (threadIdx.x == 0) part[blockIdx.x] = out[0];
+}
+
 // FP32 y/x passes with two lines per thread (fft_engine.cuh, *_pair): the
 // same 8-line tiles, tensor maps, modes and arithmetic as k_yx_tma<float,
 // float, N>, with 256 threads per tile and 128-bit exchanges, twiddle loads
@@ -326,10 +432,13 @@ __global__ void __launch_bounds__(TmaPair<N, ST, MINB>::NT, MINB)
             stage_compute_pair<N, E, +1, R0, 1>(va, vb, tws, t);
             RegChainPair<N, E, +1, LH, 1, R0, SW>::run(wk, va, vb, tws, lp, t);
         }
-        const int ca = int(g % W);
-        if (ca < VW) {
+        // MODE 0 along x runs on a caller's field (W planes, any number; no
+        // padding), where the two lines of a pair may lie in different planes
+        constexpr bool WHOLE = AXIS == 2 && MODE == 0;
+        const int ca = WHOLE ? 0 : int(g % W);
+        if (WHOLE || ca < VW) {
             const size_t b0 = AXIS == 1 ? size_t(g / W) * N * W + size_t(ca) : size_t(g);
-            const bool both = ca + 1 < VW;
+            const bool both = WHOLE || ca + 1 < VW;
 #pragma unroll
             for (int b = 0; b < E / R0; ++b)
 #pragma unroll

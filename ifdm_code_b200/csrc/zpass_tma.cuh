@@ -221,6 +221,115 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
     }
 }
 
+// ------------------------------------------------------ plain z transform ---
+// The ring of P5 around one transform of direction DIR (ifdm_fft3d and the
+// slab transforms, and the adjoint's drift): the plain one-tile-per-block kernel leaves
+// nothing in flight while it transforms (256^3 complex128, one axis pass 172 us
+// against 82 us of DRAM time).
+template <int N, int ST, int MINB, typename R, int DIR>
+__global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
+    k_fft_z_tma(cx<R> *__restrict__ data, const cx<R> *__restrict__ tw, int *__restrict__ err, int ntiles) {
+    using Z = ZT<N, R>;
+    using C = cx<R>;
+    constexpr int L = Z::L, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT5);
+    const int tid = threadIdx.x, l = tid % L, t = tid / L;
+    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT5 + 64);
+    stage_twiddles(stw, tw, N);
+    const SmemTw<C> tws{stw};
+    ring_init<ST>(bar);
+    const int my_n = ztiles_of_block(ntiles);
+    auto issue = [&](int i) {
+        const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
+        unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
+        uint64_t *b = &bar[i % ST];
+        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(C)));
+#pragma unroll 1
+        for (int r = 0; r < L; ++r)
+            bulk_load(slot + size_t(r) * Z::PP * sizeof(C), data + (row0 + r) * N, N * sizeof(C), b);
+    };
+    if (tid == 0)
+        for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
+    for (int i = 0; i < my_n; ++i) {
+        if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
+        if (!ring_wait<ST>(bar, i, my_n, err)) return;
+        unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
+        const C *lp = reinterpret_cast<const C *>(slot) + l * Z::PP;
+        C v[E];
+#pragma unroll
+        for (int b = 0; b < E / R0; ++b)
+#pragma unroll
+            for (int r = 0; r < R0; ++r) v[b * R0 + r] = lp[t + T * b + r * (N / R0)];
+        stage_compute<C, N, E, DIR, R0, 1>(v, tws, t);
+        RegChain<C, N, E, DIR, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(slot), v, tws, l, t, true);
+        C *out = data + (size_t(blockIdx.x + (long)i * gridDim.x) * L + l) * N;
+#pragma unroll
+        for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+            for (int r = 0; r < RL; ++r) out[t + T * b + r * (N / RL)] = v[b * RL + r];
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
+}
+
+// The same with two FP32 rows per thread (fft_engine.cuh, *_pair).
+template <int N, int ST, int MINB, int DIR>
+__global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
+    k_fft_z_pair(float2 *__restrict__ data, const float2 *__restrict__ tw, int *__restrict__ err, int ntiles) {
+    using Z = ZT<N>;
+    using C = float2;
+    constexpr int L = Z::L, LH = L / 2, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL;
+    static_assert(Z::NT / 2 == LH * T, "one thread per row pair");
+    extern __shared__ __align__(128) unsigned char smraw[];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT5);
+    const int tid = threadIdx.x, lp = tid % LH, t = tid / LH;
+    float4 *stw = reinterpret_cast<float4 *>(smraw + ST * Z::SLOT5 + 64);
+    stage_twiddles_staged<N>(stw, tw);
+    const StagedTw<N> tws{stw};
+    ring_init<ST>(bar);
+    const int my_n = ztiles_of_block(ntiles);
+    auto issue = [&](int i) {
+        const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
+        unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
+        uint64_t *b = &bar[i % ST];
+        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(C)));
+#pragma unroll 1
+        for (int r = 0; r < L; ++r)
+            bulk_load(slot + size_t(r) * Z::PP * sizeof(C), data + (row0 + r) * N, N * sizeof(C), b);
+    };
+    if (tid == 0)
+        for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
+    for (int i = 0; i < my_n; ++i) {
+        if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
+        if (!ring_wait<ST>(bar, i, my_n, err)) return;
+        unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
+        const C *pa = reinterpret_cast<const C *>(slot) + (2 * lp) * Z::PP, *pb = pa + Z::PP;
+        C va[E], vb[E];
+#pragma unroll
+        for (int b = 0; b < E / R0; ++b)
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                const int n = t + T * b + r * (N / R0);
+                va[b * R0 + r] = pa[n];
+                vb[b * R0 + r] = pb[n];
+            }
+        stage_compute_pair<N, E, DIR, R0, 1>(va, vb, tws, t);
+        RegChainPair<N, E, DIR, LH, 1, R0, 1>::run(reinterpret_cast<float4 *>(slot), va, vb, tws, lp, t);
+        C *oa = data + (size_t(blockIdx.x + (long)i * gridDim.x) * L + 2 * lp) * N, *ob = oa + N;
+#pragma unroll
+        for (int b = 0; b < E / RL; ++b)
+#pragma unroll
+            for (int r = 0; r < RL; ++r) {
+                const int n = t + T * b + r * (N / RL);
+                oa[n] = va[b * RL + r];
+                ob[n] = vb[b * RL + r];
+            }
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
+}
+
 // ------------------------------------------------------------------- P5 ---
 template <int N, int ST, int MINB, typename R = float>
 __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
