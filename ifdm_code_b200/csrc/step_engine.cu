@@ -200,7 +200,8 @@ template <typename R_, typename K_, int N> struct Box {
     // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
     // per SM of P1, P5 and P9
     static constexpr bool kZT = N >= 256 && std::is_same<R, K>::value;
-    static constexpr int ZST1 = 2, ZST5 = 3, ZST9 = 3, ZB1 = N >= 1024 ? 1 : 2, ZB5 = ZB1, ZB9 = ZB1;
+    static constexpr int ZST1 = 2, ZST5 = 3, ZST9 = N == 256 ? 2 : 3;
+    static constexpr int ZB1 = N >= 1024 ? 1 : (N == 256 && sizeof(C) == 16 ? 4 : 2), ZB5 = ZB1, ZB9 = ZB1;
     using ZG = ZT<(kZT ? N : 256), R>;
     // ring slots, the mbarriers (64 bytes) and the staged twiddle table
     static constexpr size_t ZSM1 = kZT ? ZST1 * ZG::SLOT1 + 64 + tw_bytes<C>(N) : 0;
@@ -214,7 +215,7 @@ template <typename R_, typename K_, int N> struct Box {
     // three slots at two blocks: the blocks overlap each other's loads; the y
     // passes at one slot and four blocks measured slower, 0.392 -> 0.43 ms;
     // at 1024 the slots leave room for one block)
-    static constexpr int ZB = N >= 1024 ? 1 : 3;
+    static constexpr int ZB = N >= 1024 ? 1 : (N == 256 ? 6 : 3);
     static constexpr int ZST1P = 1, ZB1P = ZB, ZST5P = 2, ZB5P = ZB, ZST9P = 1, ZB9P = ZB;
     static constexpr size_t ZSM1P = kZT ? ZST1P * ZG::SLOT1 + 64 + tw_bytes<C>(N) : 0;
     static constexpr size_t ZSM5P = kZT ? ZST5P * ZG::SLOT5 + 64 + tw_bytes<C>(N) : 0;
@@ -229,9 +230,9 @@ template <typename R_, typename K_, int N> struct Box {
     // (512 and 1024; at 1024 a tile takes 512 threads, one block per SM:
     // measured at 1024^3, step 57.5 -> 44.6 ms, P3 14.8 -> 8.4 ms, P5 9.0 ->
     // 6.7 ms)
-    static constexpr bool kPair = (N == 512 || N == 1024) && std::is_same<R, float>::value && std::is_same<K, float>::value;
+    static constexpr bool kPair = N >= 256 && std::is_same<R, float>::value && std::is_same<K, float>::value;
     static constexpr bool kPairZ = kPair;  // the z passes
-    static constexpr int PSTY = 2, PBY = N >= 1024 ? 1 : 3, PSTX = 2, PBX = PBY;
+    static constexpr int PSTY = 2, PBY = N >= 1024 ? 1 : (N == 256 ? 5 : 3), PSTX = 2, PBX = PBY;
     using TPY = TmaPair<(kPair ? N : 512), PSTY, PBY>;
     using TPX = TmaPair<(kPair ? N : 512), PSTX, PBX>;
     static_assert(!kPair || (TT::L == TPY::L && TX::L == TPX::L), "pair kernels share the tensor maps");

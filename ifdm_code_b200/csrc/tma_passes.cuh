@@ -34,7 +34,7 @@ template <typename R, typename K, int N, int AXIS = 1> struct TmaTile {
     // 16 lines, one block per SM).
     // 4-line x tiles, two blocks per SM at the same 128 registers (32-byte
     // TMA rows), measured slower: P3 0.92 -> 1.31 ms, P7 0.52 -> 0.59 ms.
-    static constexpr bool NARROW = !SPLIT && sizeof(G) == 8 && N >= 512;
+    static constexpr bool NARROW = !SPLIT && sizeof(G) == 8 && N >= 256;
     // FP64 y passes at N = 512: 4 lines (64-byte rows, 256 threads) so that
     // two blocks share an SM at the same 128 registers (measured: P2/P4
     // 0.89 -> 0.85 ms, P6/P8 0.50 -> 0.45 ms; the FP64 x passes measured
@@ -48,18 +48,21 @@ template <typename R, typename K, int N, int AXIS = 1> struct TmaTile {
     // threads, which spill 344 bytes a thread at 64 registers) only when
     // IFDM_NO_PAIR asks for it
     static constexpr bool BIG = N >= 1024;
+    // FP64 arithmetic at N = 256: 256-thread tiles, two slots so that three y
+    // blocks fit an SM, the x passes capped at 128 registers for two
+    static constexpr bool MID64 = sizeof(C) == 16 && N == 256;
     // resident blocks the registers must allow: two for the narrow tiles (the
     // FP32 x passes too since their twiddles come from shared memory: no
     // spills at 64 registers; measured at 512^3: P3 0.895 -> 0.877 ms, P7
     // 0.457 -> 0.433 ms)
-    static constexpr int MINB = BIG ? 1 : (NARROW || NARROW64) ? 2 : 1;
+    static constexpr int MINB = BIG ? 1 : MID64 ? (AXIS == 2 ? 3 : (SPLIT ? 3 : 2)) : (NARROW || NARROW64) ? 2 : 1;
     static constexpr int L = BIG ? (sizeof(G) == 16 ? 4 / (AXIS == 2 ? 2 : 1) : 8)
                                  : NARROW64 ? 4 : (SPLIT || NARROW) ? 8 : 128 / (int)sizeof(G);
     static constexpr bool SWZ = NARROW || NARROW64;  // slot swizzle of the exchange tile
     static constexpr int E = Plan<N>::E;
     static constexpr int T = N / E;
     static constexpr int NT = L * T;
-    static constexpr int STAGES = 3;
+    static constexpr int STAGES = MID64 && (SPLIT || AXIS == 2) ? 2 : 3;
     static constexpr int BOXR = N < 256 ? N : 256;               // rows per TMA box (limit 256)
     static constexpr size_t TILE_BYTES = size_t(N) * L * sizeof(G);
     // exchange tile between stages: the landing slot itself, or (mixed) a
