@@ -269,24 +269,19 @@ static __device__ __noinline__ void step_integrals(double ai, double max_dt, con
     const double x = c + h * gk->x[lane], wk = gk->wk[lane], wg = gk->wg[lane];
     const double x2 = x * x, x3 = x2 * x, Hx = ph.H0 * sqrt(ph.Om / x3 + (1.0 - ph.Om));
     const double f[3] = {1.0 / (Hx * x3), 1.0 / (Hx * x2), 1.0 / (Hx * (x2 * x2))};
-    double kron[3], gauss[3], sasc[3];
+    double kron[3], gauss[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         kron[q] = warp_sum(wk * f[q]);
         gauss[q] = warp_sum(wg * f[q]);
     }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) sasc[q] = warp_sum(wk * fabs(f[q] - 0.5 * kron[q])) * fabs(h);
+    // QUADPACK's estimate sasc min(1, (200 |K - G| / sasc)^1.5) is at most
+    // 200 |K - G|: where that meets the tolerance the rule is accepted without it
     int bad = 0;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        double err = fabs((kron[q] - gauss[q]) * h), r = kron[q] * h;
-        if (sasc[q] != 0.0 && err != 0.0) {
-            const double e = 200.0 * err / sasc[q], scale = e * sqrt(e);
-            err = scale < 1.0 ? sasc[q] * scale : sasc[q];
-        }
-        err = fmax(err, 50.0 * 2.220446049250313e-16 * fabs(r));  // the integrands are positive
-        if (!((err <= 1e-10 * fabs(r) && err != sasc[q]) || err == 0.0))
+        double r = kron[q] * h;
+        if (!(200.0 * fabs((kron[q] - gauss[q]) * h) <= 1e-10 * fabs(r)))
             bad |= qags_warp(q == 0 ? 3 : (q == 1 ? 2 : 4), ph.H0, ph.Om, lo, hi, ph.limit, &r);
         if (lane == 0) out->r[q] = r;
     }
