@@ -174,8 +174,12 @@ template <typename R_, typename K_, int N> struct Box {
                 CUDA_TRY(prep(k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY>, TPY::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 1, 0, PSTX, PBX>, TPX::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 2, 0, PSTX, PBX>, TPX::SMEM));
-                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, -1, PSTX, PBX>, TPX::SMEM));
-                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, +1, PSTX, PBX>, TPX::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF>, TPF::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF>, TPF::SMEM));
+                int pf = 0;
+                CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF>,
+                                                                       TPF::NT, TPF::SMEM));
+                pfgrid = sms * (pf > 0 ? pf : 1);
                 int py = 0, px = 0;
                 CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&py, k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY>,
                                                                        TPY::NT, TPY::SMEM));
@@ -235,8 +239,14 @@ template <typename R_, typename K_, int N> struct Box {
     static constexpr int PSTY = 2, PBY = N >= 1024 ? 1 : (N == 256 ? 5 : 3), PSTX = 2, PBX = PBY;
     using TPY = TmaPair<(kPair ? N : 512), PSTY, PBY>;
     using TPX = TmaPair<(kPair ? N : 512), PSTX, PBX>;
+    // one x transform of a caller's field at 512: 16 lines, 128-byte rows, one
+    // block an SM (512^3 complex64 x pass: 8 lines at three blocks 563 us, 404
+    // so; the two-transform passes are bound by their arithmetic and lost,
+    // 752 -> 819 us with the drift)
+    static constexpr int PLF = N == 512 ? 16 : 8, PBF = N == 512 ? 1 : PBX;
+    using TPF = TmaPair<(kPair ? N : 512), PSTX, PBF, PLF>;
     static_assert(!kPair || (TT::L == TPY::L && TX::L == TPX::L), "pair kernels share the tensor maps");
-    static inline int pygrid = 0, pxgrid = 0;
+    static inline int pygrid = 0, pxgrid = 0, pfgrid = 0;
     static inline int zgrid = 0;             // persistent grid of the pipelined P5
     static inline int ygrid = 0, xgrid = 0;  // persistent grids of the TMA y and x passes
 
@@ -443,16 +453,16 @@ template <typename R_, typename K_, int N> struct Box {
                 return fft_slab(data, planes, axis, sign, 0, 0, tw, s);
             }
             CUtensorMap m;
-            std::string e = make_field_map(&m, data, std::is_same<R, double>::value, N, planes, axis, axis == 1 ? TT::L : TX::L);
+            std::string e = make_field_map(&m, data, std::is_same<R, double>::value, N, planes, axis, axis == 1 ? TT::L : (kPair ? TPF::L : TX::L));
             if (!e.empty()) return e;
             if constexpr (kPair) {
-                const int nt = int(lines / TPY::L);
+                const int nt = int(lines / (axis == 1 ? TPY::L : TPF::L));
                 if (axis == 1) {
                     if (sign < 0) k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
                     else k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
                 } else {
-                    if (sign < 0) k_yx_tma_pair<N, 2, 0, -1, PSTX, PBX><<<pxgrid, TPX::NT, TPX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
-                    else k_yx_tma_pair<N, 2, 0, +1, PSTX, PBX><<<pxgrid, TPX::NT, TPX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                    if (sign < 0) k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                    else k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
                 }
             } else if (axis == 1) {
                 const int nt = int(lines / TT::L);

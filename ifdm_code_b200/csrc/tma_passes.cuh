@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(Tile<double, double, N>::NT)
 // float, N>, with 256 threads per tile and 128-bit exchanges, twiddle loads
 // shared by two lines and 16-byte global stores.  ST ring slots, MINB
 // resident blocks per SM.
-template <int N, int ST, int MINB> struct TmaPair {
-    static constexpr int L = 8, LH = L / 2;
+template <int N, int ST, int MINB, int LINES = 8> struct TmaPair {
+    static constexpr int L = LINES, LH = L / 2;
     static constexpr int E = Plan<N>::E, T = N / E, NT = LH * T;
     static constexpr int BOXR = N < 256 ? N : 256;
     static constexpr size_t TILE_BYTES = size_t(N) * L * sizeof(float2);
@@ -328,14 +328,14 @@ template <int N, int ST, int MINB> struct TmaPair {
     static_assert(SMEM <= 227 * 1024, "shared memory per block");
 };
 
-template <int N, int AXIS, int MODE, int DIR, int ST, int MINB>
-__global__ void __launch_bounds__(TmaPair<N, ST, MINB>::NT, MINB)
+template <int N, int AXIS, int MODE, int DIR, int ST, int MINB, int LINES = 8>
+__global__ void __launch_bounds__(TmaPair<N, ST, MINB, LINES>::NT, MINB)
     k_yx_tma_pair(const __grid_constant__ CUtensorMap map, float2 *__restrict__ data, int W, int VW, int ntiles,
                   TState *__restrict__ ts, const float2 *__restrict__ drift, const float2 *__restrict__ tw) {
-    using TP = TmaPair<N, ST, MINB>;
+    using TP = TmaPair<N, ST, MINB, LINES>;
     constexpr int L = TP::L, LH = TP::LH, T = TP::T, E = TP::E;
     constexpr int R0 = Plan<N>::R[0];
-    constexpr int SW = 1;  // the slot swizzle of the 8-line FP32 exchange tile (fft_engine.cuh)
+    constexpr int SW = L == 8 ? 1 : 0;  // the slot swizzle of the 8-line FP32 exchange tile (fft_engine.cuh)
     extern __shared__ __align__(128) unsigned char smraw[];
     float2 *bufs = reinterpret_cast<float2 *>(smraw);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * TP::TILE_BYTES);
