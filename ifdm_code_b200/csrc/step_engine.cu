@@ -204,8 +204,9 @@ template <typename R_, typename K_, int N> struct Box {
     // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
     // per SM of P1, P5 and P9
     static constexpr bool kZT = N >= 256 && std::is_same<R, K>::value;
-    static constexpr int ZST1 = 2, ZST5 = 3, ZST9 = N == 256 ? 2 : 3;
-    static constexpr int ZB1 = N >= 1024 ? 1 : (N == 256 && sizeof(C) == 16 ? 4 : 2), ZB5 = ZB1, ZB9 = ZB1;
+    static constexpr bool D3 = sizeof(C) == 16 && (N == 256 || N == 512);
+    static constexpr int ZST1 = D3 ? 1 : 2, ZST5 = D3 ? 2 : 3, ZST9 = D3 ? 1 : 3;
+    static constexpr int ZB1 = N >= 1024 ? 1 : (D3 ? (N == 256 ? 6 : 3) : 2), ZB5 = ZB1, ZB9 = ZB1;
     using ZG = ZT<(kZT ? N : 256), R>;
     // ring slots, the mbarriers (64 bytes) and the staged twiddle table
     static constexpr size_t ZSM1 = kZT ? ZST1 * ZG::SLOT1 + 64 + tw_bytes<C>(N) : 0;
