@@ -119,19 +119,19 @@ template <typename R_, typename K_, int N> struct Box {
             zgrid = sms * (b5 > 0 ? b5 : 1);
         }
         if constexpr (kZT) {
-            using Z = ZT<N, R>;
-            CUDA_TRY(prep(k_kick_fft_z_tma<N, ZST1, ZB1, R>, ZSM1));
-            CUDA_TRY(prep(k_density_r2c_z_tma<N, ZST5, ZB5, R>, ZSM5));
-            CUDA_TRY(prep(k_c2r_z_tma<N, ZST9, ZB9, R>, ZSM9));
+            using Z = ZT<N, R, K>;
+            CUDA_TRY(prep(k_kick_fft_z_tma<N, ZST1, ZB1, R, K>, ZSM1));
+            CUDA_TRY(prep(k_density_r2c_z_tma<N, ZST5, ZB5, R, K>, ZSM5));
+            CUDA_TRY(prep(k_c2r_z_tma<N, ZST9, ZB9, R, K>, ZSM9));
             int b1 = 0, b5 = 0, b9 = 0;
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_kick_fft_z_tma<N, ZST1, ZB1, R>, Z::NT, ZSM1));
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, k_density_r2c_z_tma<N, ZST5, ZB5, R>, Z::NT, ZSM5));
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b9, k_c2r_z_tma<N, ZST9, ZB9, R>, Z::NT, ZSM9));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_kick_fft_z_tma<N, ZST1, ZB1, R, K>, Z::NT, ZSM1));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b5, k_density_r2c_z_tma<N, ZST5, ZB5, R, K>, Z::NT, ZSM5));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b9, k_c2r_z_tma<N, ZST9, ZB9, R, K>, Z::NT, ZSM9));
             zt1grid = sms * (b1 > 0 ? b1 : 1);
             zt5grid = sms * (b5 > 0 ? b5 : 1);
             zt9grid = sms * (b9 > 0 ? b9 : 1);
-            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, -1>, ZSM5));
-            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, +1>, ZSM5));
+            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, -1>, ZSM5));
+            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, +1>, ZSM5));
             if constexpr (kPairZ) {
                 CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, -1>, ZSM5P));
                 CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, +1>, ZSM5P));
@@ -203,15 +203,15 @@ template <typename R_, typename K_, int N> struct Box {
     // z passes fed by bulk copies (zpass_tma.cuh) for N >= 256, FP32 and
     // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
     // per SM of P1, P5 and P9
-    static constexpr bool kZT = N >= 256 && std::is_same<R, K>::value;
+    static constexpr bool kZT = N >= 256 && (std::is_same<R, K>::value || N <= 512);
     static constexpr bool D3 = sizeof(C) == 16 && (N == 256 || N == 512);
     static constexpr int ZST1 = D3 ? 1 : 2, ZST5 = D3 ? 2 : 3, ZST9 = D3 ? 1 : 3;
     static constexpr int ZB1 = N >= 1024 ? 1 : (D3 ? (N == 256 ? 6 : 3) : 2), ZB5 = ZB1, ZB9 = ZB1;
-    using ZG = ZT<(kZT ? N : 256), R>;
+    using ZG = ZT<(kZT ? N : 256), R, K>;
     // ring slots, the mbarriers (64 bytes) and the staged twiddle table
-    static constexpr size_t ZSM1 = kZT ? ZST1 * ZG::SLOT1 + 64 + tw_bytes<C>(N) : 0;
-    static constexpr size_t ZSM5 = kZT ? ZST5 * ZG::SLOT5 + 64 + tw_bytes<C>(N) : 0;
-    static constexpr size_t ZSM9 = kZT ? ZST9 * ZG::SLOT9 + 64 + tw_bytes<C>(N) : 0;
+    static constexpr size_t ZSM1 = kZT ? ZST1 * ZG::SLOT1 + 64 + ZG::WORK + tw_bytes<C>(N) : 0;
+    static constexpr size_t ZSM5 = kZT ? ZST5 * ZG::SLOT5 + 64 + ZG::WORK + tw_bytes<C>(N) : 0;
+    static constexpr size_t ZSM9 = kZT ? ZST9 * ZG::SLOT9 + 64 + ZG::WORK + tw_bytes<C>(N) : 0;
     static inline int zt1grid = 0, zt5grid = 0, zt9grid = 0;  // persistent grids of the bulk-copy z passes
     // the paired z passes (two rows per thread, 256 threads at 512, 512 at
     // 1024; kPairZ below): ring slots, resident blocks per SM, shared memory
@@ -267,7 +267,7 @@ template <typename R_, typename K_, int N> struct Box {
         const unsigned nt = TL::NT;
         if constexpr (kZT) {
             if (tm && (p == 1 || p == 5 || p == 9)) {
-                using Z = ZT<N, R>;
+                using Z = ZT<N, R, K>;
                 const int nz = int(size_t(N) * N / Z::L);
                 if constexpr (kPairZ) {
                     if (std::getenv("IFDM_NO_PAIR") == nullptr) {
@@ -282,11 +282,11 @@ template <typename R_, typename K_, int N> struct Box {
                     }
                 }
                 if (p == 1)
-                    k_kick_fft_z_tma<N, ZST1, ZB1, R><<<zt1grid, Z::NT, ZSM1, s>>>(psi, phi, ts, tw, nz);
+                    k_kick_fft_z_tma<N, ZST1, ZB1, R, K><<<zt1grid, Z::NT, ZSM1, s>>>(psi, phi, ts, tw, nz);
                 else if (p == 5)
-                    k_density_r2c_z_tma<N, ZST5, ZB5, R><<<zt5grid, Z::NT, ZSM5, s>>>(psi, rhok, ts, tw, nz);
+                    k_density_r2c_z_tma<N, ZST5, ZB5, R, K><<<zt5grid, Z::NT, ZSM5, s>>>(psi, rhok, ts, tw, nz);
                 else
-                    k_c2r_z_tma<N, ZST9, ZB9, R><<<zt9grid, Z::NT, ZSM9, s>>>(rhok, phi, ts, wr, wt, tw, nz / 2);
+                    k_c2r_z_tma<N, ZST9, ZB9, R, K><<<zt9grid, Z::NT, ZSM9, s>>>(rhok, phi, ts, wr, wt, tw, nz / 2);
                 return;
             }
         }
@@ -440,14 +440,14 @@ template <typename R_, typename K_, int N> struct Box {
             const size_t lines = size_t(planes) * N;
             if (axis == 2) {
                 if constexpr (kZT) {
-                    using Z = ZT<N, R>;
+                    using Z = ZT<N, R, K>;
                     const int nz = int(lines / Z::L);
                     if constexpr (kPairZ) {
                         if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
                         else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
                     } else {
-                        if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
-                        else k_fft_z_tma<N, ZST5, ZB5, R, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
+                        if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, K, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
+                        else k_fft_z_tma<N, ZST5, ZB5, R, K, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
                     }
                     return "";
                 }

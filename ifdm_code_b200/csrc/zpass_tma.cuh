@@ -42,30 +42,35 @@ namespace ifdm {
 // rows.  Landed rows are padded by 2 elements (16 bytes FP32, 32 bytes FP64),
 // which puts the rows of a tile in different banks for the row-fastest first
 // stage.
-template <int N, typename R = float> struct ZT {
-    using C = cx<R>;
-    static constexpr int L = sizeof(R) == 4 ? 8 : 4;
+// When the arithmetic type K differs from the storage type R (mixed) the rows
+// land as they are stored and the stages exchange through a tile of their own.
+template <int N, typename R = float, typename K = R> struct ZT {
+    using G = cx<R>;
+    using C = cx<K>;
+    static constexpr bool SPLIT = !std::is_same<R, K>::value;
+    static constexpr int L = sizeof(K) == 4 ? 8 : 4;
     static constexpr int E = Plan<N>::E;
     static constexpr int T = N / E;
     static constexpr int NT = L * T;
     static constexpr int R0 = Plan<N>::R[0];
     static constexpr int RL = Plan<N>::R[Plan<N>::NST - 1];
-    static constexpr int PP = N + 2;  // complex elements per landed psi row
-    static constexpr int PF = N + 4;  // reals per landed phi row
+    static constexpr int PP = N + (SPLIT ? 4 : 2);  // complex elements per landed psi row
+    static constexpr int PF = N + (SPLIT ? 8 : 4);  // reals per landed phi row
     static constexpr int NHP = half_pitch<R>(N);
-    static constexpr int PH = NHP + 2;  // complex elements per landed half row
+    static constexpr int PH = NHP + (SPLIT ? 4 : 2);  // complex elements per landed half row
     static constexpr size_t XCH = size_t(N) * L * sizeof(C);  // [n][l] exchange tile
+    static constexpr size_t WORK = SPLIT ? XCH : 0;           // (mixed) its own place after the ring
     // P1 slot: L psi rows, then L phi rows
-    static constexpr size_t PSI_B = size_t(L) * PP * sizeof(C);
+    static constexpr size_t PSI_B = size_t(L) * PP * sizeof(G);
     static constexpr size_t SLOT1 = (PSI_B + size_t(L) * PF * sizeof(R) + 127) / 128 * 128;
     // P5 slot: L psi rows
     static constexpr size_t SLOT5 = (PSI_B + 127) / 128 * 128;
     // P9 slot: 2L half rows
-    static constexpr size_t SLOT9 = (size_t(2 * L) * PH * sizeof(C) + 127) / 128 * 128;
-    static_assert(XCH <= PSI_B && XCH <= SLOT9, "the exchange tile fits the landed rows");
+    static constexpr size_t SLOT9 = (size_t(2 * L) * PH * sizeof(G) + 127) / 128 * 128;
+    static_assert(SPLIT || (XCH <= PSI_B && XCH <= SLOT9), "the exchange tile fits the landed rows");
     static_assert(E % R0 == 0 && E % RL == 0 && R0 == RL, "register chain: equal first and last radix");
-    static_assert((N * sizeof(C)) % 16 == 0 && (NHP * sizeof(C)) % 16 == 0 && (PP * sizeof(C)) % 16 == 0 &&
-                      (PF * sizeof(R)) % 16 == 0 && (PH * sizeof(C)) % 16 == 0,
+    static_assert((N * sizeof(G)) % 16 == 0 && (NHP * sizeof(G)) % 16 == 0 && (PP * sizeof(G)) % 16 == 0 &&
+                      (PF * sizeof(R)) % 16 == 0 && (PH * sizeof(G)) % 16 == 0,
                   "bulk copies need 16-byte sizes and destinations");
 };
 
@@ -93,17 +98,18 @@ __device__ __forceinline__ int ztiles_of_block(int ntiles) {
 }
 
 // ------------------------------------------------------------------- P1 ---
-template <int N, int ST, int MINB, typename R = float>
-__global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
+template <int N, int ST, int MINB, typename R = float, typename K = R>
+__global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
     k_kick_fft_z_tma(cx<R> *__restrict__ psi, const R *__restrict__ phi, TState *__restrict__ ts,
-                     const cx<R> *__restrict__ tw, int ntiles) {
-    using Z = ZT<N, R>;
-    using C = cx<R>;
+                     const cx<K> *__restrict__ tw, int ntiles) {
+    using Z = ZT<N, R, K>;
+    using G = cx<R>;
+    using C = cx<K>;
     constexpr int L = Z::L, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL;
     extern __shared__ __align__(128) unsigned char smraw[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT1);
     const int tid = threadIdx.x, l = tid % L, t = tid / L;
-    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT1 + 64);
+    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT1 + 64 + Z::WORK);
     stage_twiddles(stw, tw, N);
     const SmemTw<C> tws{stw};
     ring_init<ST>(bar);
@@ -112,10 +118,10 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
         const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT1;
         uint64_t *b = &bar[i % ST];
-        mbar_arrive_expect_tx(b, (uint32_t)(L * N * (sizeof(C) + sizeof(R))));
+        mbar_arrive_expect_tx(b, (uint32_t)(L * N * (sizeof(G) + sizeof(R))));
 #pragma unroll 1
         for (int r = 0; r < L; ++r) {
-            bulk_load(slot + size_t(r) * Z::PP * sizeof(C), psi + (row0 + r) * N, N * sizeof(C), b);
+            bulk_load(slot + size_t(r) * Z::PP * sizeof(G), psi + (row0 + r) * N, N * sizeof(G), b);
             bulk_load(slot + Z::PSI_B + size_t(r) * Z::PF * sizeof(R), phi + (row0 + r) * N, N * sizeof(R),
                       b);
         }
@@ -123,12 +129,13 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
     if (tid == 0)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
     const double cp = ts->coefP, cq = ts->coefQ, alpha = ts->alpha;
-    const C c0 = mkc((R)ts->cre, (R)ts->cim);
+    const C c0 = mkc((K)ts->cre, (K)ts->cim);
+    const uint32_t salt = pass_salt(ts, 1);
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, &ts->err)) return;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT1;
-        const C *lp = reinterpret_cast<const C *>(slot) + l * Z::PP;
+        const G *lp = reinterpret_cast<const G *>(slot) + l * Z::PP;
         const R *lf = reinterpret_cast<const R *>(slot + Z::PSI_B) + l * Z::PF;
         C v[E];
 #pragma unroll
@@ -136,17 +143,20 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
 #pragma unroll
             for (int r = 0; r < R0; ++r) {
                 const int n = t + T * b + r * (N / R0);
-                const C g = lp[n];
+                const C g = cin<K>(lp[n]);
                 const double p = cp * (double)lf[n] + cq * (double)cnorm2(g) + alpha;
-                v[b * R0 + r] = cmul(g, expmi<R>(p)) - c0;
+                v[b * R0 + r] = cmul(g, expmi<K>(p)) - c0;
             }
         stage_compute<C, N, E, -1, R0, 1>(v, tws, t);
-        RegChain<C, N, E, -1, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(slot), v, tws, l, t, true);
-        C *out = psi + (size_t(blockIdx.x + (long)i * gridDim.x) * L + l) * N;
+        RegChain<C, N, E, -1, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(Z::SPLIT ? smraw + ST * Z::SLOT1 + 64 : slot), v, tws, l, t, true);
+        const size_t o = (size_t(blockIdx.x + (long)i * gridDim.x) * L + l) * N;
 #pragma unroll
         for (int b = 0; b < E / RL; ++b)
 #pragma unroll
-            for (int r = 0; r < RL; ++r) out[t + T * b + r * (N / RL)] = v[b * RL + r];
+            for (int r = 0; r < RL; ++r) {
+                const size_t gi = o + t + T * b + r * (N / RL);
+                psi[gi] = Cvt<R, K>::out(v[b * RL + r], salt, gi);
+            }
         fence_proxy_async_smem();
         __syncthreads();
     }
@@ -226,16 +236,17 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
 // slab transforms, and the adjoint's drift): the plain one-tile-per-block kernel leaves
 // nothing in flight while it transforms (256^3 complex128, one axis pass 172 us
 // against 82 us of DRAM time).
-template <int N, int ST, int MINB, typename R, int DIR>
-__global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
-    k_fft_z_tma(cx<R> *__restrict__ data, const cx<R> *__restrict__ tw, int *__restrict__ err, int ntiles) {
-    using Z = ZT<N, R>;
-    using C = cx<R>;
+template <int N, int ST, int MINB, typename R, typename K, int DIR>
+__global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
+    k_fft_z_tma(cx<R> *__restrict__ data, const cx<K> *__restrict__ tw, int *__restrict__ err, int ntiles) {
+    using Z = ZT<N, R, K>;
+    using G = cx<R>;
+    using C = cx<K>;
     constexpr int L = Z::L, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL;
     extern __shared__ __align__(128) unsigned char smraw[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT5);
     const int tid = threadIdx.x, l = tid % L, t = tid / L;
-    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT5 + 64);
+    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT5 + 64 + Z::WORK);
     stage_twiddles(stw, tw, N);
     const SmemTw<C> tws{stw};
     ring_init<ST>(bar);
@@ -244,10 +255,10 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
         const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
         uint64_t *b = &bar[i % ST];
-        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(C)));
+        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(G)));
 #pragma unroll 1
         for (int r = 0; r < L; ++r)
-            bulk_load(slot + size_t(r) * Z::PP * sizeof(C), data + (row0 + r) * N, N * sizeof(C), b);
+            bulk_load(slot + size_t(r) * Z::PP * sizeof(G), data + (row0 + r) * N, N * sizeof(G), b);
     };
     if (tid == 0)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
@@ -255,19 +266,22 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, err)) return;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
-        const C *lp = reinterpret_cast<const C *>(slot) + l * Z::PP;
+        const G *lp = reinterpret_cast<const G *>(slot) + l * Z::PP;
         C v[E];
 #pragma unroll
         for (int b = 0; b < E / R0; ++b)
 #pragma unroll
-            for (int r = 0; r < R0; ++r) v[b * R0 + r] = lp[t + T * b + r * (N / R0)];
+            for (int r = 0; r < R0; ++r) v[b * R0 + r] = cin<K>(lp[t + T * b + r * (N / R0)]);
         stage_compute<C, N, E, DIR, R0, 1>(v, tws, t);
-        RegChain<C, N, E, DIR, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(slot), v, tws, l, t, true);
-        C *out = data + (size_t(blockIdx.x + (long)i * gridDim.x) * L + l) * N;
+        RegChain<C, N, E, DIR, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(Z::SPLIT ? smraw + ST * Z::SLOT5 + 64 : slot), v, tws, l, t, true);
+        const size_t o = (size_t(blockIdx.x + (long)i * gridDim.x) * L + l) * N;
 #pragma unroll
         for (int b = 0; b < E / RL; ++b)
 #pragma unroll
-            for (int r = 0; r < RL; ++r) out[t + T * b + r * (N / RL)] = v[b * RL + r];
+            for (int r = 0; r < RL; ++r) {
+                const size_t gi = o + t + T * b + r * (N / RL);
+                data[gi] = Cvt<R, K>::out(v[b * RL + r], 0x2545f491u, gi);
+            }
         fence_proxy_async_smem();
         __syncthreads();
     }
@@ -331,19 +345,20 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
 }
 
 // ------------------------------------------------------------------- P5 ---
-template <int N, int ST, int MINB, typename R = float>
-__global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
+template <int N, int ST, int MINB, typename R = float, typename K = R>
+__global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
     k_density_r2c_z_tma(cx<R> *__restrict__ psi, cx<R> *__restrict__ rhok, TState *__restrict__ ts,
-                        const cx<R> *__restrict__ tw, int ntiles) {
-    using Z = ZT<N, R>;
-    using C = cx<R>;
+                        const cx<K> *__restrict__ tw, int ntiles) {
+    using Z = ZT<N, R, K>;
+    using G = cx<R>;
+    using C = cx<K>;
     constexpr int L = Z::L, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL, NT = Z::NT;
     constexpr int M = N / 2, NHP = Z::NHP;
     constexpr int LH = L / 2;  // packed complex lines of the density transform
     extern __shared__ __align__(128) unsigned char smraw[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT5);
     const int tid = threadIdx.x, l = tid % L, t = tid / L;
-    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT5 + 64);
+    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT5 + 64 + Z::WORK);
     stage_twiddles(stw, tw, N);
     const SmemTw<C> tws{stw};
     // the density transform: 4 lines, T threads each (whole warps: threads < LH * T)
@@ -355,48 +370,50 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
         const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
         uint64_t *b = &bar[i % ST];
-        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(C)));
+        mbar_arrive_expect_tx(b, (uint32_t)(L * N * sizeof(G)));
 #pragma unroll 1
         for (int r = 0; r < L; ++r)
-            bulk_load(slot + size_t(r) * Z::PP * sizeof(C), psi + (row0 + r) * N, N * sizeof(C), b);
+            bulk_load(slot + size_t(r) * Z::PP * sizeof(G), psi + (row0 + r) * N, N * sizeof(G), b);
     };
     if (tid == 0)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
     const double mu = ts->mu;
-    const C c0 = mkc((R)ts->cre, (R)ts->cim);
+    const C c0 = mkc((K)ts->cre, (K)ts->cim);
+    const uint32_t salt = pass_salt(ts, 5), salt2 = pass_salt(ts, 10);
     double mx = 0.0;
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, &ts->err)) return;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
-        C *wk = reinterpret_cast<C *>(slot);
+        C *wk = reinterpret_cast<C *>(Z::SPLIT ? smraw + ST * Z::SLOT5 + 64 : slot);
         const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * L;
         // inverse FFT of psi along z, stage 0 from the landed rows
         C v[E];
-        const C *lp = reinterpret_cast<const C *>(slot) + l * Z::PP;
+        const G *lp = reinterpret_cast<const G *>(slot) + l * Z::PP;
 #pragma unroll
         for (int b = 0; b < E / R0; ++b)
 #pragma unroll
-            for (int r = 0; r < R0; ++r) v[b * R0 + r] = lp[t + T * b + r * (N / R0)];
+            for (int r = 0; r < R0; ++r) v[b * R0 + r] = cin<K>(lp[t + T * b + r * (N / R0)]);
         stage_compute<C, N, E, +1, R0, 1>(v, tws, t);
         RegChain<C, N, E, +1, L, L, 1, R0, 1>::run(wk, v, tws, l, t, true);
         // psi = IFFT + c; rho = |psi|^2 - mu into a real tile that pairs rows
         // p and p+LH of element n: rt[(n*LH + p)*2 + h] holds row p + h*LH
         // (conflict-free stores of the [l, t] layout and complex loads of the
         // packed layout)
-        R rho[E];
-        C *out = psi + (row0 + l) * N;
+        K rho[E];
+        const size_t o = (row0 + l) * N;
 #pragma unroll
         for (int b = 0; b < E / RL; ++b)
 #pragma unroll
             for (int r = 0; r < RL; ++r) {
-                const C g = v[b * RL + r] + c0;
-                out[t + T * b + r * (N / RL)] = g;
-                const double n2 = (double)cnorm2(g);
+                const size_t gi = o + t + T * b + r * (N / RL);
+                const G g = Cvt<R, K>::out(v[b * RL + r] + c0, salt, gi);
+                psi[gi] = g;
+                const double n2 = (double)cnorm2(cin<K>(g));  // the stored value defines the density
                 mx = fmax(mx, n2);
-                rho[b * RL + r] = (R)(n2 - mu);
+                rho[b * RL + r] = (K)(n2 - mu);
             }
-        R *rt = reinterpret_cast<R *>(slot);
+        K *rt = reinterpret_cast<K *>(wk);
         __syncthreads();  // every thread is done with the exchange tile
 #pragma unroll
         for (int b = 0; b < E / RL; ++b)
@@ -427,10 +444,11 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
             const int pp = q % LH, k = q / LH;
             const C zk = wk[k * LH + pp];
             const C zc = cconj(wk[((N - k) % N) * LH + pp]);
-            const C s = cscale(zk + zc, R(0.5));
-            const C d = cscale(zk - zc, R(0.5));
-            rhok[(row0 + pp) * NHP + k] = s;
-            rhok[(row0 + pp + LH) * NHP + k] = mkc(d.y, -d.x);
+            const C s = cscale(zk + zc, K(0.5));
+            const C d = cscale(zk - zc, K(0.5));
+            const size_t ga = (row0 + pp) * NHP + k, gb = ga + size_t(LH) * NHP;
+            rhok[ga] = Cvt<R, K>::out(s, salt2, ga);
+            rhok[gb] = Cvt<R, K>::out(mkc(d.y, -d.x), salt2, gb);
         }
         fence_proxy_async_smem();
         __syncthreads();
@@ -545,18 +563,19 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
 }
 
 // ------------------------------------------------------------------- P9 ---
-template <int N, int ST, int MINB, typename R = float>
-__global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
+template <int N, int ST, int MINB, typename R = float, typename K = R>
+__global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
     k_c2r_z_tma(const cx<R> *__restrict__ rhok, R *__restrict__ phi, TState *__restrict__ ts, long win_rows,
-                int win_tail, const cx<R> *__restrict__ tw, int ntiles) {
-    using Z = ZT<N, R>;
-    using C = cx<R>;
+                int win_tail, const cx<K> *__restrict__ tw, int ntiles) {
+    using Z = ZT<N, R, K>;
+    using G = cx<R>;
+    using C = cx<K>;
     constexpr int L = Z::L, T = Z::T, E = Z::E, R0 = Z::R0, RL = Z::RL;
     constexpr int M = N / 2, NHP = Z::NHP, ROWS = 2 * L;
     extern __shared__ __align__(128) unsigned char smraw[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + ST * Z::SLOT9);
     const int tid = threadIdx.x, l = tid % L, t = tid / L;
-    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT9 + 64);
+    C *stw = reinterpret_cast<C *>(smraw + ST * Z::SLOT9 + 64 + Z::WORK);
     stage_twiddles(stw, tw, N);
     const SmemTw<C> tws{stw};
     ring_init<ST>(bar);
@@ -565,21 +584,22 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
         const size_t row0 = size_t(blockIdx.x + (long)i * gridDim.x) * ROWS;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT9;
         uint64_t *b = &bar[i % ST];
-        mbar_arrive_expect_tx(b, (uint32_t)(ROWS * NHP * sizeof(C)));
+        mbar_arrive_expect_tx(b, (uint32_t)(ROWS * NHP * sizeof(G)));
 #pragma unroll 1
         for (int r = 0; r < ROWS; ++r)
-            bulk_load(slot + size_t(r) * Z::PH * sizeof(C), rhok + (row0 + r) * NHP, NHP * sizeof(C), b);
+            bulk_load(slot + size_t(r) * Z::PH * sizeof(G), rhok + (row0 + r) * NHP, NHP * sizeof(G), b);
     };
     if (tid == 0)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
-    constexpr KSplit<R> inv(1.0 / ((double)N * N * N));
+    const uint32_t salt = pass_salt(ts, 9);
+    constexpr KSplit<K> inv(1.0 / ((double)N * N * N));
     double mx = 0.0;  // the running max on the FP64 pipe, which this pass leaves idle
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, &ts->err)) return;
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT9;
-        const C *xa = reinterpret_cast<const C *>(slot) + l * Z::PH;
-        const C *xb = xa + L * Z::PH;
+        const G *xa = reinterpret_cast<const G *>(slot) + l * Z::PH;
+        const G *xb = xa + L * Z::PH;
         C v[E];
 #pragma unroll
         for (int bb = 0; bb < E / R0; ++bb)
@@ -587,15 +607,15 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
             for (int r = 0; r < R0; ++r) {
                 const int n = t + T * bb + r * (N / R0);
                 const int m = n <= M ? n : N - n;
-                C a = xa[m], b = xb[m];
+                C a = cin<K>(xa[m]), b = cin<K>(xb[m]);
                 if (m == 0 || m == M) {  // c2r ignores these imaginary parts
-                    a.y = R(0);
-                    b.y = R(0);
+                    a.y = K(0);
+                    b.y = K(0);
                 }
                 v[bb * R0 + r] = n <= M ? mkc(a.x - b.y, a.y + b.x) : mkc(a.x + b.y, b.x - a.y);
             }
         stage_compute<C, N, E, +1, R0, 1>(v, tws, t);
-        RegChain<C, N, E, +1, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(slot), v, tws, l, t, true);
+        RegChain<C, N, E, +1, L, L, 1, R0, 1>::run(reinterpret_cast<C *>(Z::SPLIT ? smraw + ST * Z::SLOT9 + 64 : slot), v, tws, l, t, true);
         const long ra = long(blockIdx.x + (long)i * gridDim.x) * ROWS + l, rb = ra + L;
         // elements of rows below win_rows, and the first win_tail of row win_rows, are in the window
         const int lima = ra < win_rows ? N : (ra == win_rows ? win_tail : 0);
@@ -607,7 +627,8 @@ __global__ void __launch_bounds__(ZT<N, R>::NT, MINB)
             for (int r = 0; r < RL; ++r) {
                 const int n = t + T * bb + r * (N / RL);
                 const C z = v[bb * RL + r];
-                const R fa = mulk(z.x, inv.hi, inv.lo), fb = mulk(z.y, inv.hi, inv.lo);
+                const R fa = Cvt<R, K>::outr(mulk(z.x, inv.hi, inv.lo), salt, size_t(ra) * N + n);
+                const R fb = Cvt<R, K>::outr(mulk(z.y, inv.hi, inv.lo), salt, size_t(rb) * N + n);
                 oa[n] = fa;
                 ob[n] = fb;
                 if (n < lima) mx = fmax(mx, fabs((double)fa));
