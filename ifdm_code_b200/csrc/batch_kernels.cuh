@@ -1,4 +1,6 @@
-// batch_kernels.cuh -- many independent boxes advanced by one persistent kernel.
+// batch_kernels.cuh -- many independent boxes whose plane does not fit a CTA
+// (128^3 in FP64 arithmetic) advanced by one persistent kernel; all smaller
+// boxes run the plane kernels of box_kernels.cuh.
 //
 // The work of a step of box b is a list of items: the timestep (one item),
 // then the tiles of passes P1..P9 (the same fused passes as step_kernels.cuh,
@@ -355,7 +357,7 @@ template <typename R, typename K, int N, class P> struct BatchOps {
 // the launch has size N.  Launches of different sizes run side by side.
 template <typename R, typename K, int N, int V>
 __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
-    using Ops = BatchOps<R, K, N, PlanV<N, V>>;
+    using Ops = BatchOps<R, K, N, Plan<N>>;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ long long s_item;
     __shared__ int s_ok;
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
 template <typename R, typename K, int N, int V, int PH>
 __global__ void __launch_bounds__(kBatchThreads) k_batch_phase(const BatchBox *boxes) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    BatchOps<R, K, N, PlanV<N, V>>::template phase<PH>(smraw, boxes[blockIdx.y], (int)blockIdx.x);
+    BatchOps<R, K, N, Plan<N>>::template phase<PH>(smraw, boxes[blockIdx.y], (int)blockIdx.x);
 }
 
 }  // namespace ifdm

@@ -65,14 +65,6 @@ template <> struct Plan<512> { static constexpr int E = 8, NST = 3; static const
 // (chained transforms) with 8 elements per thread
 template <> struct Plan<1024> { static constexpr int E = 8, NST = 4; static constexpr int R[4] = {4, 8, 8, 4}; };
 
-// Alternative radix orders with the same elements per thread (V = 1), for the
-// batch autotuner; V = 0 and sizes without an alternative are Plan<N>.
-template <int N, int V> struct PlanV : Plan<N> {};
-template <> struct PlanV<32, 1> { static constexpr int E = 8, NST = 2; static constexpr int R[2] = {4, 8}; };
-template <> struct PlanV<48, 1> { static constexpr int E = 12, NST = 3; static constexpr int R[3] = {3, 4, 4}; };
-template <> struct PlanV<64, 1> { static constexpr int E = 8, NST = 3; static constexpr int R[3] = {4, 4, 4}; };
-template <> struct PlanV<96, 1> { static constexpr int E = 12, NST = 4; static constexpr int R[4] = {3, 4, 2, 4}; };
-
 // ------------------------------------------------------------- butterflies --
 template <int RAD, int DIR> struct Bfly;
 

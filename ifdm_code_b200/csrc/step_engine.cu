@@ -203,10 +203,10 @@ template <typename R_, typename K_, int N> struct Box {
     // z passes fed by bulk copies (zpass_tma.cuh) for N >= 256, FP32 and
     // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
     // per SM of P1, P5 and P9
-    static constexpr bool kZT = N >= 256 && (std::is_same<R, K>::value || N <= 512);
-    static constexpr bool D3 = sizeof(C) == 16 && (N == 256 || N == 512);
+    static constexpr bool kZT = (N >= 256 && (std::is_same<R, K>::value || N <= 512)) || (N == 128 && sizeof(K) == 8);
+    static constexpr bool D3 = sizeof(C) == 16 && N >= 128 && N <= 512;
     static constexpr int ZST1 = D3 ? 1 : 2, ZST5 = D3 ? 2 : 3, ZST9 = D3 ? 1 : 3;
-    static constexpr int ZB1 = N >= 1024 ? 1 : (D3 ? (N == 256 ? 6 : 3) : 2), ZB5 = ZB1, ZB9 = ZB1;
+    static constexpr int ZB1 = N >= 1024 ? 1 : (D3 ? 3 * 512 / N : 2), ZB5 = ZB1, ZB9 = ZB1;
     using ZG = ZT<(kZT ? N : 256), R, K>;
     // ring slots, the mbarriers (64 bytes) and the staged twiddle table
     static constexpr size_t ZSM1 = kZT ? ZST1 * ZG::SLOT1 + 64 + ZG::WORK + tw_bytes<C>(N) : 0;
@@ -353,14 +353,36 @@ template <typename R_, typename K_, int N> struct Box {
         k_reduce_init<<<1, 256, 0, s>>>(ts, part, (int)zrows(), double(N) * N * N);
     }
 
+    // One transform along z of `rows` rows: the ring-fed kernels where the base
+    // is 16-byte aligned (bulk copies), else the plain one.
+    static void z_pass(cudaStream_t s, G *data, size_t rows, int sign, const C *tw, uint32_t salt, bool ring) {
+        if constexpr (kZT) {
+            if (ring) {
+                using Z = ZT<N, R, K>;
+                const int nz = int(rows / Z::L);
+                if constexpr (kPairZ) {
+                    if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
+                    else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
+                } else {
+                    if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, K, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz, salt);
+                    else k_fft_z_tma<N, ZST5, ZB5, R, K, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz, salt);
+                }
+                return;
+            }
+        }
+        const unsigned gz = unsigned(rows / TZ::L);
+        if (sign < 0) k_fft_z<R, K, N, -1><<<gz, TZ::NT, SMZ, s>>>(data, tw, salt);
+        else k_fft_z<R, K, N, +1><<<gz, TZ::NT, SMZ, s>>>(data, tw, salt);
+    }
+
     // g <- U^H g: forward FFT, drift with the conjugate tables, inverse FFT
     static void adj_drift(cudaStream_t s, G *g, TState *ts_adj, const C *drift_conj, const C *tw,
                           const CUtensorMap *tm, uint32_t salt) {
-        k_fft_z<R, K, N, -1><<<zrows(), TZ::NT, SMZ, s>>>(g, tw, salt);
+        z_pass(s, g, size_t(N) * N, -1, tw, salt, tm != nullptr);
         pass(2, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
         pass(3, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
         pass(4, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
-        k_fft_z<R, K, N, +1><<<zrows(), TZ::NT, SMZ, s>>>(g, tw, salt ^ 0x68e31da4u);
+        z_pass(s, g, size_t(N) * N, +1, tw, salt ^ 0x68e31da4u, tm != nullptr);
     }
     // pw = phi_s[w]: real source -> half spectrum -> -1/kappa^2 -> real
     static void poisson_of(cudaStream_t s, const R *w, R *pw, G *rhok, TState *ts_adj, const C *tw, const C *twh,
@@ -414,10 +436,9 @@ template <typename R_, typename K_, int N> struct Box {
     static std::string fft_slab(G *data, int planes, int axis, int sign, int op, int y0, const C *tw, cudaStream_t s) {
         const size_t nl = size_t(planes) * N;
         if (nl % TL::L || nl % TZ::L) return "planes * n must be a multiple of the tile lines";
-        const unsigned gz = unsigned(nl / TZ::L), gl = unsigned(nl / TL::L), nt = TL::NT;
+        const unsigned gl = unsigned(nl / TL::L), nt = TL::NT;
         if (axis == 2) {
-            if (sign < 0) k_fft_z<R, K, N, -1><<<gz, TZ::NT, SMZ, s>>>(data, tw, 0x2545f491u);
-            else k_fft_z<R, K, N, +1><<<gz, TZ::NT, SMZ, s>>>(data, tw, 0x2545f491u);
+            z_pass(s, data, nl, sign, tw, 0x2545f491u, false);
         } else if (axis == 1) {
             if (sign < 0) k_fft_yx<R, K, N, -1, 1><<<gl, nt, SM, s>>>(data, N, N, nullptr, 0, tw);
             else k_fft_yx<R, K, N, +1, 1><<<gl, nt, SM, s>>>(data, N, N, nullptr, 0, tw);
@@ -439,19 +460,8 @@ template <typename R_, typename K_, int N> struct Box {
         if constexpr (kFftTma) {
             const size_t lines = size_t(planes) * N;
             if (axis == 2) {
-                if constexpr (kZT) {
-                    using Z = ZT<N, R, K>;
-                    const int nz = int(lines / Z::L);
-                    if constexpr (kPairZ) {
-                        if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
-                        else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
-                    } else {
-                        if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, K, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
-                        else k_fft_z_tma<N, ZST5, ZB5, R, K, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz);
-                    }
-                    return "";
-                }
-                return fft_slab(data, planes, axis, sign, 0, 0, tw, s);
+                z_pass(s, data, lines, sign, tw, 0x2545f491u, true);
+                return "";
             }
             CUtensorMap m;
             std::string e = make_field_map(&m, data, std::is_same<R, double>::value, N, planes, axis, axis == 1 ? TT::L : (kPair ? TPF::L : TX::L));

@@ -50,12 +50,12 @@ template <typename R, typename K, int N, int AXIS = 1> struct TmaTile {
     static constexpr bool BIG = N >= 1024;
     // FP64 arithmetic at N = 256: 256-thread tiles, two slots so that three y
     // blocks fit an SM, the x passes capped at 128 registers for two
-    static constexpr bool MID64 = sizeof(C) == 16 && N == 256;
+    static constexpr bool MID64 = sizeof(C) == 16 && N <= 256;
     // resident blocks the registers must allow: two for the narrow tiles (the
     // FP32 x passes too since their twiddles come from shared memory: no
     // spills at 64 registers; measured at 512^3: P3 0.895 -> 0.877 ms, P7
     // 0.457 -> 0.433 ms)
-    static constexpr int MINB = BIG ? 1 : MID64 ? (AXIS == 2 ? 3 : (SPLIT ? 3 : 2)) : (NARROW || NARROW64) ? 2 : 1;
+    static constexpr int MINB = BIG ? 1 : MID64 ? (AXIS == 2 || SPLIT ? 3 : 2) * 256 / N : (NARROW || NARROW64) ? 2 : 1;
     static constexpr int L = BIG ? (sizeof(G) == 16 ? 4 / (AXIS == 2 ? 2 : 1) : 8)
                                  : NARROW64 ? 4 : (SPLIT || NARROW) ? 8 : 128 / (int)sizeof(G);
     static constexpr bool SWZ = NARROW || NARROW64;  // slot swizzle of the exchange tile

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
 // against 82 us of DRAM time).
 template <int N, int ST, int MINB, typename R, typename K, int DIR>
 __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
-    k_fft_z_tma(cx<R> *__restrict__ data, const cx<K> *__restrict__ tw, int *__restrict__ err, int ntiles) {
+    k_fft_z_tma(cx<R> *__restrict__ data, const cx<K> *__restrict__ tw, int *__restrict__ err, int ntiles, uint32_t salt) {
     using Z = ZT<N, R, K>;
     using G = cx<R>;
     using C = cx<K>;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
 #pragma unroll
             for (int r = 0; r < RL; ++r) {
                 const size_t gi = o + t + T * b + r * (N / RL);
-                data[gi] = Cvt<R, K>::out(v[b * RL + r], 0x2545f491u, gi);
+                data[gi] = Cvt<R, K>::out(v[b * RL + r], salt, gi);
             }
         fence_proxy_async_smem();
         __syncthreads();

@@ -89,3 +89,25 @@ def test_diagnostics_against_numpy(n, prec):
     for q, w in want.items():
         assert e[q] == pytest.approx(w, rel=1e-11), q
     assert ps["mean_rho"] == pytest.approx(rho.mean(), rel=1e-12)
+
+
+@pytest.mark.parametrize("n,prec", [(128, "fp64"), (128, "mixed"), (256, "fp64"), (256, "fp32"), (256, "mixed")])
+def test_adjoint_on_ring_passes(n, prec, monkeypatch):
+    # the adjoint drift's z transforms on the ring-fed kernels against the plain
+    # ones: a step and its adjoint are 12 transforms each, three steps, every
+    # transform to TOL
+    psi0 = zeldovich_psi(n, seed=n)
+    rng = np.random.default_rng(n)
+    cot = rng.standard_normal((n,) * 3) + 1j * rng.standard_normal((n,) * 3)
+    out = []
+    for plain in (False, True):
+        if plain:
+            monkeypatch.setenv("IFDM_NO_TMA", "1")
+        else:
+            monkeypatch.delenv("IFDM_NO_TMA", raising=False)
+        with ifdm.Simulation(2.5e-24, 0.0, 5.0, n, precision=prec) as s:
+            s.set_psi(psi0, 1.0 / 51.0)
+            s.record_steps(3, 0.01, 2)
+            out.append(np.empty_like(cot))
+            s.adjoint(cot, out[-1])
+    assert np.linalg.norm(out[0] - out[1]) <= 72 * TOL[prec] * np.linalg.norm(out[1])
