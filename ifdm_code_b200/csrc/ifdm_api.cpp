@@ -647,11 +647,23 @@ template <class F> static int for_each_box(ifdm_batch *b, F fn) {
     return IFDM_OK;
 }
 
+// box i's launches while other boxes of its size run their own
+struct SharedDevice {
+    StepEngine &eng;
+    SharedDevice(ifdm_batch *b, int i) : eng(b->ctx[i]->eng) {
+        int same = 0;
+        for (ifdm_ctx *c : b->ctx) same += c->N == b->ctx[i]->N;
+        eng.share_device(same > 1);
+    }
+    ~SharedDevice() { eng.share_device(false); }
+};
+
 extern "C" {
 
 int ifdm_batch_record_steps(ifdm_batch *b, int nsteps, const double *dt_scale, int checkpoint_every) {
     if (!b || nsteps <= 0 || !dt_scale || checkpoint_every <= 0) return IFDM_ERR_ARGS;
     return for_each_box(b, [&](int i) {
+        SharedDevice sd(b, i);
         const int rc = ifdm_record_steps(b->ctx[i], nsteps, dt_scale[i], checkpoint_every);
         return rc ? rc : ifdm_synchronize(b->ctx[i]);
     });
@@ -659,7 +671,10 @@ int ifdm_batch_record_steps(ifdm_batch *b, int nsteps, const double *dt_scale, i
 
 int ifdm_batch_adjoint(ifdm_batch *b, const double *const *g_final, double *const *g0) {
     if (!b || !g_final || !g0) return IFDM_ERR_ARGS;
-    return for_each_box(b, [&](int i) { return ifdm_adjoint(b->ctx[i], g_final[i], g0[i]); });
+    return for_each_box(b, [&](int i) {
+        SharedDevice sd(b, i);
+        return ifdm_adjoint(b->ctx[i], g_final[i], g0[i]);
+    });
 }
 
 int ifdm_batch_info(ifdm_batch *b, long long *items_per_step, int *grid) {

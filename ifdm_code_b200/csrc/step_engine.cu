@@ -722,11 +722,11 @@ std::string StepEngine::init_box() {
     // 1000-2000 cycles against 3000 of the counter in global memory), else a cooperative grid
     box_group_ = N;
     box_cluster_ = N <= 16;
-    bool runs = false;
+    int resident = 0;
     {
         // attributes and the occupancy query once per device, size and precision
         std::lock_guard<std::mutex> lk(setup_mutex());
-        static std::map<std::array<int, 3>, bool> known;
+        static std::map<std::array<int, 3>, int> known;
         int dev = 0;
         CUDA_TRY(cudaGetDevice(&dev));
         const std::array<int, 3> key{dev, N, cfg_.precision};
@@ -734,13 +734,28 @@ std::string StepEngine::init_box() {
         if (it == known.end()) {
             std::string e = bk.setup(N, 0);
             if (!e.empty()) return e;
-            it = known.emplace(key, bk.resident(N, box_group_, box_cluster_) >= 1).first;
+            it = known.emplace(key, bk.resident(N, box_group_, box_cluster_)).first;
         }
-        runs = it->second;
+        resident = it->second;
     }
-    box_ = runs && std::getenv("IFDM_NO_FUSE") == nullptr;
+    box_half_ = resident == 1 && !box_cluster_;
+    box_ = resident >= 1 && std::getenv("IFDM_NO_FUSE") == nullptr;
     CUDA_TRY(cudaMalloc(&box_scr_, sizeof(BoxScratch)));
     CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
+    return "";
+}
+
+// Several boxes of this size step at the same time.  Where the device holds one
+// group of N CTAs (96^3, FP32 128^3: a CTA an SM), the boxes would take turns
+// and 52 of 148 SMs idle: groups of N/2 with two planes a CTA let two or three
+// boxes run side by side, which costs one box time (a step's phases double, its
+// barriers do not), so only then.  The results do not depend on the group.
+std::string StepEngine::share_device(bool on) {
+    const int group = on && box_half_ ? cfg_.N / 2 : cfg_.N;
+    if (!box_ || group == box_group_) return "";
+    // the barrier's counter is a multiple of the group when a launch starts
+    CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
+    box_group_ = group;
     return "";
 }
 

@@ -69,6 +69,7 @@ class StepEngine {
     // Adjoint support.  record(): nsteps fixed-mode steps that keep a per-step
     // log of the coefficients and a checkpoint of (psi, phi) every ckpt steps.
     std::string record(int nsteps, double dt_scale, int ckpt);
+    std::string share_device(bool on);  // other boxes of this size run at the same time
     // gradient of a real loss through the recorded steps: g_final = dL/dpsi_final
     // (complex128, natural units, dL/dRe + i dL/dIm) -> g0 = dL/dpsi_0; both
     // device pointers.  Leaves the context's state at an intermediate step.
@@ -124,6 +125,7 @@ class StepEngine {
     // adjoint buffers
     // one-launch box kernels (box_kernels.cuh): N <= 128 where a plane fits
     bool box_ = false, box_cluster_ = false;
+    bool box_half_ = false;    // one group of N CTAs fills the device (share_device)
     int box_group_ = 0;        // CTAs of the group that runs this box
     void *box_scr_ = nullptr;  // BoxScratch
     std::string init_box();

@@ -124,3 +124,32 @@ def test_two_boxes_in_flight_on_two_streams(n):
             a.step(4, 0.01)
             b.step(4, 0.01)
         assert np.array_equal(a.get_psi(), alone[0]) and np.array_equal(b.get_psi(), alone[1])
+
+
+@pytest.mark.parametrize("prec,n", [("fp32", 96), ("fp64", 96), ("mixed", 96), ("fp32", 128)])
+def test_batch_record_in_half_groups(prec, n):
+    # boxes that fill the device alone record and sweep with two planes a CTA
+    # when a batch holds several: the same bits as one box by itself
+    psis = [zeldovich_psi(n, seed=n + i) for i in range(3)]
+    rng = np.random.default_rng(n)
+    cot = [rng.standard_normal((n,) * 3) + 1j * rng.standard_normal((n,) * 3) for _ in psis]
+    want = []
+    sims = [ifdm.Simulation(MFDM, 0.0, XMAX, n, precision=prec) for _ in psis]
+    for s, p, c in zip(sims, psis, cot):
+        s.set_psi(p, A0)
+        s.record_steps(5, 0.01, 2)
+        psi, g = s.get_psi(), np.empty_like(c)
+        s.adjoint(c, g)
+        want.append((psi, g))
+        s.set_psi(p, A0)
+    got = [np.empty_like(c) for c in cot]
+    with ifdm.Batch(sims) as b:
+        b.record_steps(5, 0.01, 2)
+        psi = [s.get_psi() for s in sims]
+        b.adjoint(cot, got)
+    for i, s in enumerate(sims):
+        assert np.array_equal(psi[i], want[i][0]) and np.array_equal(got[i], want[i][1]), i
+        s.set_psi(psis[i], A0)
+        s.step(5, 0.01)  # whole groups again
+        assert s.state()["device_error"] == 0 and np.array_equal(s.get_psi(), want[i][0]), i
+        s.close()
