@@ -200,9 +200,12 @@ template <typename R_, typename K_, int N> struct Box {
     static constexpr bool kTma = N >= 128;
     static constexpr bool kFftTma = N >= 256;  // the callers' own fields (axis_pass)
     static constexpr bool kZPipe = N >= 128 && N <= 512 && std::is_same<R, float>::value && std::is_same<K, float>::value;
-    // z passes fed by bulk copies (zpass_tma.cuh) for N >= 256, FP32 and
-    // FP64 (8 FP32 or 4 FP64 rows per tile); ring depth and resident blocks
-    // per SM of P1, P5 and P9
+    // z passes fed by bulk copies (zpass_tma.cuh) for N >= 256 and, in FP64
+    // arithmetic, 128 (8 FP32 or 4 FP64 rows per tile; FP32 at 128 runs the
+    // box kernels); ring depth and resident blocks per SM of P1, P5 and P9.
+    // D3: one slot (two in P5) and three blocks at 512, six at 256, twelve at
+    // 128: the blocks hide each other's loads (FP64 512^3 step 7.42 -> 7.31 ms
+    // against two or three slots at two blocks; 256^3 873 -> 862 us)
     static constexpr bool kZT = (N >= 256 && (std::is_same<R, K>::value || N <= 512)) || (N == 128 && sizeof(K) == 8);
     static constexpr bool D3 = sizeof(C) == 16 && N >= 128 && N <= 512;
     static constexpr int ZST1 = D3 ? 1 : 2, ZST5 = D3 ? 2 : 3, ZST9 = D3 ? 1 : 3;

@@ -48,8 +48,13 @@ template <typename R, typename K, int N, int AXIS = 1> struct TmaTile {
     // threads, which spill 344 bytes a thread at 64 registers) only when
     // IFDM_NO_PAIR asks for it
     static constexpr bool BIG = N >= 1024;
-    // FP64 arithmetic at N = 256: 256-thread tiles, two slots so that three y
-    // blocks fit an SM, the x passes capped at 128 registers for two
+    // FP64 arithmetic at N <= 256 (128-byte rows: 256 threads a tile at N =
+    // 256, 128 at N = 128): the two-transform x passes and mixed's passes keep
+    // two slots and 85 registers for three (six) blocks an SM, the FP64 y
+    // passes three slots and two (four) blocks.  Uncapped (162 registers) one
+    // block was resident: 256^3 P3 186 -> 151 us; 128^3 step 155 -> 145 us
+    // together with the bulk-copy z passes.  N = 512 keeps one 512-thread
+    // block: 4-line tiles measured slower there (above).
     static constexpr bool MID64 = sizeof(C) == 16 && N <= 256;
     // resident blocks the registers must allow: two for the narrow tiles (the
     // FP32 x passes too since their twiddles come from shared memory: no

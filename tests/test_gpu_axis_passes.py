@@ -111,3 +111,21 @@ def test_adjoint_on_ring_passes(n, prec, monkeypatch):
             out.append(np.empty_like(cot))
             s.adjoint(cot, out[-1])
     assert np.linalg.norm(out[0] - out[1]) <= 72 * TOL[prec] * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("n", [256, 512])
+def test_two_rows_per_thread_same_bits(n, monkeypatch):
+    # FP32 from 256 points on: two lines a thread, the arithmetic of the
+    # one-line kernels
+    psi0 = zeldovich_psi(n, seed=n)
+    out = []
+    for plain in (False, True):
+        if plain:
+            monkeypatch.setenv("IFDM_NO_PAIR", "1")
+        else:
+            monkeypatch.delenv("IFDM_NO_PAIR", raising=False)
+        with ifdm.Simulation(2.5e-24, 1e-63, 5.0, n, precision="fp32") as s:
+            s.set_psi(psi0, 1.0 / 51.0)
+            s.step(4, 0.01)
+            out.append((s.get_psi(), s.get_phi()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
