@@ -221,8 +221,8 @@ def supported_res(res: int, precision: str = "fp64") -> bool:
 class Batch:
     """Several Simulations (res 16..128, one device, one precision) advanced
     together: one replay of a captured CUDA graph per ``step`` call, in which
-    the boxes of each grid size share one persistent kernel (or one launch per
-    phase, whichever ``tune`` found faster).  Each box keeps its own state and
+    the boxes of each grid size share one kernel for all steps (a cluster of
+    CTAs per box, small boxes) or one launch per phase.  Each box keeps its own state and
     is read through its Simulation as usual."""
 
     def __init__(self, sims: list[Simulation]):

@@ -199,9 +199,8 @@ int ifdm_adjoint(ifdm_ctx *ctx, const double *g_final, double *g0);
  * ifdm_load_snapshot).  ifdm_batch_step advances every box by nsteps
  * fixed-mode steps, box b with step scale dt_scale[b] (as ifdm_step), in one
  * replay of one captured CUDA graph: the boxes of each grid size share one
- * persistent kernel (or, the other schedule, one launch per phase), sizes run
- * side by side, with the same passes and tile shapes as a one-box run of
- * these sizes.  Contexts are read as usual afterwards (ifdm_get_psi,
+ * kernel for all steps (a cluster of CTAs per box) or one launch per phase,
+ * sizes run side by side, with the same phases as a one-box run of these sizes.  Contexts are read as usual afterwards (ifdm_get_psi,
  * ifdm_get_state) and must outlive the batch.  ifdm_batch_tune times launch
  * shapes on trial_steps steps (saving and restoring every box's state) and
  * keeps the fastest: the schedule, CTAs per SM, the group size of the item
@@ -209,7 +208,7 @@ int ifdm_adjoint(ifdm_ctx *ctx, const double *g_final, double *g0);
  * radix plan of each grid size. */
 typedef struct ifdm_batch ifdm_batch;
 typedef struct ifdm_batch_tuning {
-    int mode;           /* 0: one persistent kernel per grid size, 1: one launch per phase and size */
+    int mode;           /* 0: one kernel per grid size where that is the faster, 1: one launch per phase and size */
     int blocks_per_sm;  /* persistent CTAs per SM */
     int group;          /* boxes per group of the item order, 0 = all boxes */
     int plan[6];        /* radix-plan variant (0, 1) for res 16, 32, 48, 64, 96, 128 */
