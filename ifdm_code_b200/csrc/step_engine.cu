@@ -650,6 +650,7 @@ StepEngine::~StepEngine() {
     cudaFree(ts_adj_);
     cudaFree(drift64_adj_);
     cudaFree(drift32_adj_);
+    if (ev_read_) cudaEventDestroy(ev_read_);
     if (copy_stream_) cudaStreamSynchronize(copy_stream_);
     for (int s = 0; s < 2; ++s) {
         cudaFree(stage_[s]);
@@ -686,6 +687,7 @@ std::string StepEngine::init(const EngineConfig &cfg, cudaStream_t stream) {
     CUDA_TRY(cudaMalloc(&drift32_, sizeof(float2) * N));
     CUDA_TRY(cudaMalloc(&ts_, sizeof(TState)));
     CUDA_TRY(cudaMemsetAsync(ts_, 0, sizeof(TState), stream_));
+    CUDA_TRY(cudaEventCreateWithFlags(&ev_read_, cudaEventDisableTiming));
     std::string e = get_twiddles(N, compute_kind(cfg.precision), &tw_);
     if (!e.empty()) return e;
     e = get_twiddles(N / 2, compute_kind(cfg.precision), &twh_);
@@ -847,6 +849,7 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         else k_psi_in<float><<<1184, 256, 0, stream_>>>((const double2 *)psi, (float2 *)psi_, invS, n3);
 
         CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaEventRecord(ev_read_, stream_));
     } else {
         // chunk i: host -> slot i%2 on the copy stream, then the conversion on
         // the compute stream; the copy of chunk i+1 runs during conversion i,
@@ -891,9 +894,15 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         l.stream = stream_;
         CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
         CUDA_TRY(box_kernels(prec).load(cfg_.N, l, a0));
-        return "";
+        if (on_device) CUDA_TRY(cudaEventRecord(ev_read_, stream_));
+    } else {
+        std::string e = launch_initial_density();
+        if (!e.empty()) return e;
     }
-    return launch_initial_density();
+    // stream_ may still hold earlier steps: the caller's tensor is free for
+    // reuse on any stream only once the kernel that reads it has run
+    if (on_device) CUDA_TRY(cudaEventSynchronize(ev_read_));
+    return "";
 }
 
 std::string StepEngine::psi_to_host(double *host_out, int which) {

@@ -48,7 +48,8 @@ class StepEngine {
     // Allocates device buffers on the current device; returns "" or an error.
     std::string init(const EngineConfig &cfg, cudaStream_t stream);
     // psi (host or device complex128, N^3) -> scaled state; sets a and rho_c,
-    // runs the initial density/Poisson passes.  Asynchronous.
+    // runs the initial density/Poisson passes, asynchronously; returns once psi
+    // has been read.
     std::string load_psi(const double *psi_c128, bool on_device, double a, double rhoc);
     // nsteps fixed-mode steps (timestep + 9 passes each).  Asynchronous.
     std::string step(int nsteps, double dt_scale);
@@ -106,6 +107,7 @@ class StepEngine {
     double2 *stage_[2] = {nullptr, nullptr};
     cudaStream_t copy_stream_ = nullptr;
     cudaEvent_t ev_copied_[2] = {nullptr, nullptr}, ev_free_[2] = {nullptr, nullptr};
+    cudaEvent_t ev_read_ = nullptr;  // after the kernel that reads a caller's device psi
 
     EngineConfig cfg_{};
     cudaStream_t stream_ = nullptr;

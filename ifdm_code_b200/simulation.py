@@ -83,7 +83,10 @@ class Simulation:
         self._c(self.lib.ifdm_load_snapshot(self.h, t))
 
     def set_psi(self, psi, a: float, rhoc: float = 0.0) -> None:
-        """psi: complex128 array (host numpy) or CUDA tensor of N^3 elements."""
+        """psi: complex128 array (host numpy) or CUDA tensor of N^3 elements.  A
+        tensor is read on the box's own stream: its values must be complete
+        (synchronise the stream that computes them first); it may be overwritten
+        once the call returns."""
         if hasattr(psi, "data_ptr"):
             ptr = psi.data_ptr()
             self._c(self.lib.ifdm_set_psi(self.h, C.c_void_p(ptr), a, rhoc))

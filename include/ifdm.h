@@ -108,8 +108,10 @@ int ifdm_supported_res(int res, int precision);
 int ifdm_load_ic(ifdm_ctx *ctx);
 /* read_rerun (src/gadget_IC.h:709-750): psi and a from <icpath>output<t>.dat. */
 int ifdm_load_snapshot(ifdm_ctx *ctx, int t);
-/* Start from a host psi (complex128, N^3) at scale factor a; rhoc <= 0 means
- * the constant 3.51059e10 that read_rerun uses. */
+/* Start from psi (complex128, N^3, host or device) at scale factor a; rhoc <= 0
+ * means the constant 3.51059e10 that read_rerun uses.  A device psi must be
+ * complete (the context reads it on its own stream); when the call returns psi
+ * has been read and may be overwritten or freed. */
 int ifdm_set_psi(ifdm_ctx *ctx, const double *psi, double a, double rhoc);
 /* psi after the latest full step (the pending second half-kick applied). */
 int ifdm_get_psi(ifdm_ctx *ctx, double *psi);
