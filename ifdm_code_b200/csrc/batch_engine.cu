@@ -111,7 +111,7 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
         }
     }
     CUDA_TRY(cudaMalloc(&d_status_, sizeof(int)));
-    CUDA_TRY(cudaMemset(d_status_, 0, sizeof(int)));
+    CUDA_TRY(cudaMemsetAsync(d_status_, 0, sizeof(int), stream_));
     ev_.resize(boxes_.size(), nullptr);
     for (auto &e : ev_) CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CUDA_TRY(cudaEventCreateWithFlags(&ev_done_, cudaEventDisableTiming));
@@ -178,7 +178,9 @@ std::string BatchEngine::prepare(const double *dt_scale) {
         Class &c = cls_[ci];
         const int nb = (int)c.boxes.size();
         const int V = knobs.plan[batch_size_index(c.N)] ? 1 : 0;
-        CUDA_TRY(cudaMemcpy(c.d_boxes, hb[ci].data(), hb[ci].size(), cudaMemcpyHostToDevice));
+        // on the batch's own stream: an earlier step still in flight reads these
+        // tables, and the next launch must not run before they have landed
+        CUDA_TRY(cudaMemcpyAsync(c.d_boxes, hb[ci].data(), hb[ci].size(), cudaMemcpyHostToDevice, stream_));
         if (c.box) {
             c.grid = c.group * nb;
             c.step_items = 0;
@@ -203,7 +205,7 @@ std::string BatchEngine::prepare(const double *dt_scale) {
                 }
         c.nsegs = (int)segs.size();
         c.step_items = first;
-        CUDA_TRY(cudaMemcpy(c.d_segs, segs.data(), sizeof(BatchSeg) * segs.size(), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(c.d_segs, segs.data(), sizeof(BatchSeg) * segs.size(), cudaMemcpyHostToDevice, stream_));
     }
     for (auto &g : graphs_) cudaGraphExecDestroy(g.second);
     graphs_.clear();

@@ -158,3 +158,30 @@ def test_batch_adjoint_equals_each_box(prec):
             want = np.empty_like(g0[i])
             sim.adjoint(gfin[i], want)
         assert np.array_equal(g0[i], want), i
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_batch_steps_of_other_sizes_queued_behind_each_other(mode):
+    # the second call rewrites the boxes' tables (step scales) while the first
+    # call's steps are in flight: the same bits as with a wait between them
+    sims, psis, dts = _boxes("fp64")
+    other = [0.5 * d for d in dts]
+    out = []
+    with ifdm.Batch(sims) as b:
+        b.set_tuning(mode=mode, blocks_per_sm=2, group=3 if mode == 0 else 0)
+        for wait in (True, False):
+            for s, p in zip(sims, psis):
+                s.set_psi(p, A0)
+            b.step(20, dts)
+            if wait:
+                b.synchronize()
+            b.step(10, other)
+            if wait:
+                b.synchronize()
+            b.step(10, dts)
+            b.synchronize()
+            out.append([s.get_psi() for s in sims])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+    for s in sims:
+        s.close()
