@@ -616,6 +616,9 @@ static std::string get_twiddles(int n, int prec, void **out) {
         CUDA_TRY(cudaMalloc(&p, sizeof(float2) * t.size()));
         CUDA_TRY(cudaMemcpy(p, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
     }
+    // a copy from pageable memory may return before it has landed, and the
+    // kernels run on streams that do not order themselves against its stream
+    CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
     cache.push_back({dev, n, prec, p});
     *out = p;
     return "";
