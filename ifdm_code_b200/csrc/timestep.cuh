@@ -311,6 +311,7 @@ static __device__ __noinline__ void timestep_warp(TState *ts, const Phys &ph, co
     if (max_dt > dt_PE) { max_dt = dt_PE; crit = 2; }
     if ((max_dt > dt_QI) && (ph.g != 0)) { max_dt = dt_QI; crit = 4; }
     if (crit != 3) step_integrals(ai, max_dt, ph, gk, si);
+    __syncwarp();  // every lane has read *ts and *si before lane 0 rewrites *ts
     if ((threadIdx.x & 31) != 0) return;
     if (si->bad) ts->err |= 1;
     ts->maxphi = maxphi;
