@@ -37,6 +37,8 @@ namespace ifdm {
 
 namespace {
 
+const char *const kGaveUp = "a device-side wait gave up";
+
 constexpr int kBinBlocks = 592, kBinThreads = 256;  // 4 blocks per SM
 constexpr int kBinWarps = kBinThreads / 32;
 
@@ -278,13 +280,16 @@ std::string field_means(const EngineView &v, double S, double2 *field, double *w
     });
     for (int axis = 1; e.empty() && axis >= 0; --axis) {
         int np = 0;
-        e = axis_k2(field, N, axis, work + off_axis(N), &np, s);
+        e = axis_k2(field, N, axis, work + off_axis(N), &np, &v.ts->err, s);
         if (e.empty()) k_sum_cols<<<1, 1024, 0, s>>>(work + off_axis(N), np, 1, 1, tot + 4 + axis);
     }
     if (!e.empty()) return e;
     double h[6];
+    int err = 0;
     DG_TRY(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, s));
+    DG_TRY(cudaMemcpyAsync(&err, &v.ts->err, sizeof(err), cudaMemcpyDeviceToHost, s));
     DG_TRY(cudaStreamSynchronize(s));
+    if (err & 2) return kGaveUp;
     const double S2 = S * S, kf = 3.14159265358979323846 / xmax;  // k = pi kappa / xmax
     out[0] = h[0] / n3 * S2;
     // Parseval per axis: sum_x |d psi/dz|^2 = sum over lines of sum_k k^2 |.|^2 / N
@@ -330,15 +335,18 @@ std::string power_spectrum(const EngineView &v, double S, double2 *field, double
         if (v.precision == 0) return go(k_rho_half_z<double, decltype(n)::value>, (const double2 *)v.psi);
         return go(k_rho_half_z<float, decltype(n)::value>, (const float2 *)v.psi);
     });
-    if (e.empty()) e = fft_half_axis(field, N, 1, s);
-    if (e.empty()) e = fft_half_axis(field, N, 0, s);
+    if (e.empty()) e = fft_half_axis(field, N, 1, v.ts, s);
+    if (e.empty()) e = fft_half_axis(field, N, 0, v.ts, s);
     if (!e.empty()) return e;
     k_bin_half<<<kBinBlocks, kBinThreads, 0, s>>>(field, N, half_pitch<double>(N), nbins, ed, work + off_bins(N));
     k_bin_total<<<nbins, 256, 0, s>>>(work + off_bins(N), kBinBlocks, nbins, tot);
     DG_TRY(cudaGetLastError());
     std::vector<double> h(3 * kMaxBins + 1);
+    int err = 0;
     DG_TRY(cudaMemcpyAsync(h.data(), tot, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
+    DG_TRY(cudaMemcpyAsync(&err, &v.ts->err, sizeof(err), cudaMemcpyDeviceToHost, s));
     DG_TRY(cudaStreamSynchronize(s));
+    if (err & 2) return kGaveUp;
     const double mean = h[3 * kMaxBins] / n3;
     if (mean_rho) *mean_rho = mean * S * S;
     // delta_k = rho_k / mean for kappa != 0 (the bins exclude kappa = 0)

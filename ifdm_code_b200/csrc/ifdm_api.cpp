@@ -213,15 +213,19 @@ int ifdm_get_phi(ifdm_ctx *c, double *phi) {
     return IFDM_OK;
 }
 
+static int diag_code(const std::string &e, int other) {
+    return e.find("gave up") != std::string::npos ? IFDM_ERR_DEVICE : other;
+}
+
 int ifdm_power_spectrum(ifdm_ctx *c, int nbins, const double *edges, double *k, double *pk, long long *modes,
                         double *mean_rho) {
     if (!c || nbins < 1 || nbins > kMaxBins) return fail(c, IFDM_ERR_ARGS, "nbins must be 1..64");
     if (!c->have_psi) return fail(c, IFDM_ERR_STATE, "no wave function loaded");
     if (ensure_out(c) || ensure_diag(c)) return IFDM_ERR_CUDA;
     if (c->snap.ready()) CTX_STR(c, IFDM_ERR_CUDA, c->snap.before_stage(c->stream));
-    CTX_STR(c, IFDM_ERR_ARGS, power_spectrum(c->eng.view(), c->eng.S(), reinterpret_cast<double2 *>(c->d_out), c->d_diag,
-                                             2.0 * c->xmax, nbins, edges, k, pk, modes, mean_rho, c->stream));
-    return IFDM_OK;
+    const std::string e = power_spectrum(c->eng.view(), c->eng.S(), reinterpret_cast<double2 *>(c->d_out), c->d_diag,
+                                         2.0 * c->xmax, nbins, edges, k, pk, modes, mean_rho, c->stream);
+    return e.empty() ? IFDM_OK : fail(c, diag_code(e, IFDM_ERR_ARGS), e);
 }
 
 int ifdm_get_energies(ifdm_ctx *c, ifdm_energies *out) {
@@ -230,8 +234,9 @@ int ifdm_get_energies(ifdm_ctx *c, ifdm_energies *out) {
     if (ensure_out(c) || ensure_diag(c)) return IFDM_ERR_CUDA;
     if (c->snap.ready()) CTX_STR(c, IFDM_ERR_CUDA, c->snap.before_stage(c->stream));
     double m[4];
-    CTX_STR(c, IFDM_ERR_CUDA, field_means(c->eng.view(), c->eng.S(), reinterpret_cast<double2 *>(c->d_out), c->d_diag,
-                                          c->xmax, m, c->stream));
+    const std::string e = field_means(c->eng.view(), c->eng.S(), reinterpret_cast<double2 *>(c->d_out), c->d_diag, c->xmax,
+                                      m, c->stream);
+    if (!e.empty()) return fail(c, diag_code(e, IFDM_ERR_CUDA), e);
     m[2] *= c->eng.Phi0();  // phi is stored in units of Phi0
     out->mean_rho = m[0];
     out->mean_grad2 = m[1];
@@ -523,9 +528,9 @@ int ifdm_adjoint(ifdm_ctx *c, const double *g_final, double *g0) {
     cudaError_t ce = cudaStreamSynchronize(c->stream);
     if (e.empty() && ce != cudaSuccess) e = std::string("cudaStreamSynchronize: ") + cudaGetErrorString(ce);
     if (!e.empty()) return fail(c, IFDM_ERR_CUDA, e);
-    TState t{};
-    CTX_STR(c, IFDM_ERR_CUDA, c->eng.read_state(t));
-    if (t.err) return fail(c, IFDM_ERR_DEVICE, "a device-side check failed during the adjoint");
+    int err = 0;
+    CTX_STR(c, IFDM_ERR_CUDA, c->eng.adjoint_error(err));
+    if (err) return fail(c, IFDM_ERR_DEVICE, "a device-side check failed during the adjoint");
     return IFDM_OK;
 }
 

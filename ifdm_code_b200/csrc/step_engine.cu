@@ -358,17 +358,17 @@ template <typename R_, typename K_, int N> struct Box {
 
     // One transform along z of `rows` rows: the ring-fed kernels where the base
     // is 16-byte aligned (bulk copies), else the plain one.
-    static void z_pass(cudaStream_t s, G *data, size_t rows, int sign, const C *tw, uint32_t salt, bool ring) {
+    static void z_pass(cudaStream_t s, G *data, size_t rows, int sign, const C *tw, uint32_t salt, bool ring, int *err) {
         if constexpr (kZT) {
             if (ring) {
                 using Z = ZT<N, R, K>;
                 const int nz = int(rows / Z::L);
                 if constexpr (kPairZ) {
-                    if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
-                    else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, nullptr, nz);
+                    if (sign < 0) k_fft_z_pair<N, ZST5P, ZB5P, -1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, err, nz);
+                    else k_fft_z_pair<N, ZST5P, ZB5P, +1><<<zt5pgrid, Z::NT / 2, ZSM5P, s>>>(data, tw, err, nz);
                 } else {
-                    if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, K, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz, salt);
-                    else k_fft_z_tma<N, ZST5, ZB5, R, K, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, nullptr, nz, salt);
+                    if (sign < 0) k_fft_z_tma<N, ZST5, ZB5, R, K, -1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, err, nz, salt);
+                    else k_fft_z_tma<N, ZST5, ZB5, R, K, +1><<<zt5grid, Z::NT, ZSM5, s>>>(data, tw, err, nz, salt);
                 }
                 return;
             }
@@ -381,11 +381,11 @@ template <typename R_, typename K_, int N> struct Box {
     // g <- U^H g: forward FFT, drift with the conjugate tables, inverse FFT
     static void adj_drift(cudaStream_t s, G *g, TState *ts_adj, const C *drift_conj, const C *tw,
                           const CUtensorMap *tm, uint32_t salt) {
-        z_pass(s, g, size_t(N) * N, -1, tw, salt, tm != nullptr);
+        z_pass(s, g, size_t(N) * N, -1, tw, salt, tm != nullptr, &ts_adj->err);
         pass(2, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
         pass(3, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
         pass(4, s, g, nullptr, nullptr, ts_adj, drift_conj, tw, nullptr, 0, 0, tm);
-        z_pass(s, g, size_t(N) * N, +1, tw, salt ^ 0x68e31da4u, tm != nullptr);
+        z_pass(s, g, size_t(N) * N, +1, tw, salt ^ 0x68e31da4u, tm != nullptr, &ts_adj->err);
     }
     // pw = phi_s[w]: real source -> half spectrum -> -1/kappa^2 -> real
     static void poisson_of(cudaStream_t s, const R *w, R *pw, G *rhok, TState *ts_adj, const C *tw, const C *twh,
@@ -398,16 +398,17 @@ template <typename R_, typename K_, int N> struct Box {
     // x-slab [planes][N][N], axis 1 = y on the x-slab, axis 0 = x on the
     // transposed y-slab [N][planes][N] (op 1: forward, -1/(kappa^2 N^3) with
     // global y offset y0, inverse).
-    // Forward pass along axis 1 (y) or 0 (x) of a half spectrum [N][N][NHP] (diagnostics; FP64)
-    static std::string half_axis(G *data, int axis, const C *tw, cudaStream_t s) {
+    // Forward pass along axis 1 (y) or 0 (x) of a half spectrum [N][N][NHP]
+    // (diagnostics; FP64); a wait that gives up sets ts->err
+    static std::string half_axis(G *data, int axis, const C *tw, TState *ts, cudaStream_t s) {
         if constexpr (kFftTma && std::is_same<R, double>::value) {
             CUtensorMap my, mx;
             std::string e = make_axis_maps(&my, &mx, data, true, N, NHP, TT::L, TX::L, N < 256 ? N : 256);
             if (!e.empty()) return e;
             if (axis == 1)
-                k_yx_tma<R, K, N, 1, 0, -1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, data, NHP, NH, int(size_t(N) * NHP / TT::L), nullptr, 6, nullptr, tw);
+                k_yx_tma<R, K, N, 1, 0, -1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, data, NHP, NH, int(size_t(N) * NHP / TT::L), ts, 6, nullptr, tw);
             else
-                k_yx_tma<R, K, N, 2, 0, -1><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, data, NHP, NH, int(size_t(N) * NHP / TX::L), nullptr, 7, nullptr, tw);
+                k_yx_tma<R, K, N, 2, 0, -1><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, data, NHP, NH, int(size_t(N) * NHP / TX::L), ts, 7, nullptr, tw);
         } else if (axis == 1) {
             k_fft_yx<R, K, N, -1, 1><<<hblocks(), TL::NT, SM, s>>>(data, NHP, NH, nullptr, 0, tw);
         } else {
@@ -417,7 +418,7 @@ template <typename R_, typename K_, int N> struct Box {
     }
     // sum of kappa^2 |.|^2 over the forward transforms along axis 1 or 0 of a
     // field [N][N][N] (diagnostics; FP64): one partial sum a block, *nparts of them
-    static std::string line_k2(const G *data, int axis, double *part, int *nparts, const C *tw, cudaStream_t s) {
+    static std::string line_k2(const G *data, int axis, double *part, int *nparts, const C *tw, int *err, cudaStream_t s) {
         if constexpr (std::is_same<R, double>::value) {
             if constexpr (kFftTma) {
                 CUtensorMap my, mx;
@@ -425,8 +426,8 @@ template <typename R_, typename K_, int N> struct Box {
                 if (!e.empty()) return e;
                 const int nt = int(size_t(N) * N / (axis == 1 ? TT::L : TX::L));
                 *nparts = axis == 1 ? ygrid : xgrid;
-                if (axis == 1) k_line_k2_tma<N, 1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, nt, tw, part);
-                else k_line_k2_tma<N, 2><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, nt, tw, part);
+                if (axis == 1) k_line_k2_tma<N, 1><<<ygrid, TT::NT, TT::SMEM, s>>>(my, nt, tw, part, err);
+                else k_line_k2_tma<N, 2><<<xgrid, TX::NT, TX::SMEM, s>>>(mx, nt, tw, part, err);
             } else {
                 *nparts = int(zblocks());
                 if (axis == 1) k_line_k2<N, 1><<<zblocks(), TL::NT, SM, s>>>(data, tw, part);
@@ -441,7 +442,7 @@ template <typename R_, typename K_, int N> struct Box {
         if (nl % TL::L || nl % TZ::L) return "planes * n must be a multiple of the tile lines";
         const unsigned gl = unsigned(nl / TL::L), nt = TL::NT;
         if (axis == 2) {
-            z_pass(s, data, nl, sign, tw, 0x2545f491u, false);
+            z_pass(s, data, nl, sign, tw, 0x2545f491u, false, nullptr);
         } else if (axis == 1) {
             if (sign < 0) k_fft_yx<R, K, N, -1, 1><<<gl, nt, SM, s>>>(data, N, N, nullptr, 0, tw);
             else k_fft_yx<R, K, N, +1, 1><<<gl, nt, SM, s>>>(data, N, N, nullptr, 0, tw);
@@ -463,7 +464,7 @@ template <typename R_, typename K_, int N> struct Box {
         if constexpr (kFftTma) {
             const size_t lines = size_t(planes) * N;
             if (axis == 2) {
-                z_pass(s, data, lines, sign, tw, 0x2545f491u, true);
+                z_pass(s, data, lines, sign, tw, 0x2545f491u, true, nullptr);
                 return "";
             }
             CUtensorMap m;
@@ -1072,6 +1073,15 @@ std::string StepEngine::read_state(TState &out) {
 }
 
 // ------------------------------------------------------------------ adjoint --
+std::string StepEngine::adjoint_error(int &err) {
+    int e[2] = {0, 0};
+    CUDA_TRY(cudaMemcpyAsync(&e[0], &ts_->err, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    if (!box_) CUDA_TRY(cudaMemcpyAsync(&e[1], &ts_adj_->err, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    CUDA_TRY(cudaStreamSynchronize(stream_));
+    err = e[0] | e[1];
+    return "";
+}
+
 std::string StepEngine::ensure_adjoint_buffers(int nsteps, int ckpt) {
     const size_t n3 = n3_();
     const size_t rs = storage_bytes(cfg_.precision), cs = 2 * rs;
@@ -1173,6 +1183,7 @@ std::string StepEngine::adjoint_kick(void *psi, void *phi, double a, double aP, 
 
 std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
     if (recorded_ <= 0) return "adjoint: no recorded steps";
+    if (!box_) CUDA_TRY(cudaMemsetAsync(ts_adj_, 0, sizeof(TState), stream_));
     const size_t n3 = n3_();
     const size_t rs = storage_bytes(cfg_.precision), cs = 2 * rs;
     const int M = recorded_, K = ckpt_every_;
@@ -1361,14 +1372,14 @@ template <typename F> static std::string with_fp64(int n, F &&f) {
         return "";
     });
 }
-std::string fft_half_axis(void *data, int n, int axis, cudaStream_t stream) {
+std::string fft_half_axis(void *data, int n, int axis, TState *ts, cudaStream_t stream) {
     return with_fp64(n, [&](auto box, const double2 *tw) {
-        return decltype(box)::half_axis((double2 *)data, axis, tw, stream);
+        return decltype(box)::half_axis((double2 *)data, axis, tw, ts, stream);
     });
 }
-std::string axis_k2(const void *data, int n, int axis, double *part, int *nparts, cudaStream_t stream) {
+std::string axis_k2(const void *data, int n, int axis, double *part, int *nparts, int *err, cudaStream_t stream) {
     return with_fp64(n, [&](auto box, const double2 *tw) {
-        return decltype(box)::line_k2((const double2 *)data, axis, part, nparts, tw, stream);
+        return decltype(box)::line_k2((const double2 *)data, axis, part, nparts, tw, err, stream);
     });
 }
 std::string twiddle_tables(int n, int precision, const void **tw, const void **twh) {

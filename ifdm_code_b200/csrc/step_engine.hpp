@@ -75,6 +75,8 @@ class StepEngine {
     // (complex128, natural units, dL/dRe + i dL/dIm) -> g0 = dL/dpsi_0; both
     // device pointers.  Leaves the context's state at an intermediate step.
     std::string adjoint(const double *g_final_dev, double *g0_dev);
+    // error bits of the replay and of the backward sweep (synchronous)
+    std::string adjoint_error(int &err);
     int recorded_steps() const { return recorded_; }
     // one step split for the native loop: timestep only / passes only
     std::string timestep_only(double dt_scale);
@@ -153,11 +155,12 @@ std::string fft3d(void *data, int n, int precision, int sign, cudaStream_t strea
 // One axis of a slab-decomposed 3-D FFT on device data (ifdm_fft_slab).
 std::string fft_slab(void *data, int n, int planes, int axis, int precision, int sign, int op, int y0,
                      cudaStream_t stream);
-// Forward FP64 pass along axis 1 (y) or 0 (x) of a half spectrum [n][n][half_pitch].
-std::string fft_half_axis(void *data, int n, int axis, cudaStream_t stream);
+// Forward FP64 pass along axis 1 (y) or 0 (x) of a half spectrum [n][n][half_pitch];
+// bit 2 of ts->err is set when a device wait gives up.
+std::string fft_half_axis(void *data, int n, int axis, TState *ts, cudaStream_t stream);
 // Sum over the lines along axis 1 or 0 of an FP64 field [n][n][n] of kappa^2 |transform|^2:
-// *nparts (at most n^2 / 2) partial sums in part.
-std::string axis_k2(const void *data, int n, int axis, double *part, int *nparts, cudaStream_t stream);
+// *nparts (at most n^2 / 2) partial sums in part; bit 2 of *err as above.
+std::string axis_k2(const void *data, int n, int axis, double *part, int *nparts, int *err, cudaStream_t stream);
 // Device tables of n and n/2 points in a precision mode's arithmetic type.
 std::string twiddle_tables(int n, int precision, const void **tw, const void **twh);
 bool supported_n(int n);

@@ -7,7 +7,8 @@
 //
 // Every wait is bounded: after kMaxSpins polls (with nanosleep back-off, well
 // over a second in total) the waiter records an error in *err and returns
-// false instead of spinning forever.
+// false instead of spinning forever.  Transforms of a caller's field have no
+// error word: they fill what they gave up with NaN.
 #pragma once
 
 #include <cuda.h>
@@ -16,7 +17,10 @@
 
 namespace ifdm {
 
-constexpr uint32_t kMaxSpins = 1u << 24;
+#ifndef IFDM_MAX_SPINS
+#define IFDM_MAX_SPINS (1u << 24)
+#endif
+constexpr uint32_t kMaxSpins = IFDM_MAX_SPINS;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -59,6 +63,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
     }
     if (err) atomicOr(err, flag);
     return false;
+}
+
+// NaN into elements first, first + stride, ... (count of them) of a field of
+// complex numbers, all threads of the block: the lines a kernel without an
+// error word gave up
+template <typename G> __device__ __noinline__ void fill_nan(G *data, size_t first, size_t stride, int count) {
+    const float q = __int_as_float(0x7fffffff);
+    G v;
+    v.x = q;
+    v.y = q;
+    for (int n = threadIdx.x; n < count; n += blockDim.x) data[first + n * stride] = v;
 }
 
 // generic-proxy accesses to shared memory before later async-proxy writes

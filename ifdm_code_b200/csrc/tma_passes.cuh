@@ -136,6 +136,11 @@ __global__ void __launch_bounds__(TmaTile<R, K, N, AXIS>::NT, TmaTile<R, K, N, A
                 for (int j = i; j < my_n && j <= i + ST - 1; ++j)
                     mbar_wait(&bar[j % ST], (uint32_t)((j / ST) & 1), err, 2);
             __syncthreads();
+            if (MODE == 0 && !err)  // a caller's field
+                for (long q = 0; q < long(my_n - i) * L; ++q) {
+                    const long gl = ((long)blockIdx.x + (i + q / L) * (long)gridDim.x) * L + q % L;
+                    if (gl % W < VW) fill_nan(data, AXIS == 1 ? size_t(gl / W) * N * W + size_t(gl % W) : size_t(gl), S, N);
+                }
             return;
         }
         const long g = ((long)blockIdx.x + (long)i * gridDim.x) * L + l;
@@ -217,7 +222,7 @@ __global__ void __launch_bounds__(TmaTile<R, K, N, AXIS>::NT, TmaTile<R, K, N, A
 template <int N, int AXIS>
 __global__ void __launch_bounds__(TmaTile<double, double, N, AXIS>::NT, TmaTile<double, double, N, AXIS>::MINB)
     k_line_k2_tma(const __grid_constant__ CUtensorMap map, int ntiles, const double2 *__restrict__ tw,
-                  double *__restrict__ part) {
+                  double *__restrict__ part, int *__restrict__ err) {
     using TL = TmaTile<double, double, N, AXIS>;
     using C = double2;
     constexpr int L = TL::L, T = TL::T, ST = TL::STAGES, E = TL::E;
@@ -253,12 +258,12 @@ __global__ void __launch_bounds__(TmaTile<double, double, N, AXIS>::NT, TmaTile<
     for (int i = 0; i < my_n; ++i) {
         const int s = i % ST;
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
-        const bool ok = mbar_wait(&bar[s], (uint32_t)((i / ST) & 1), nullptr, 2);
+        const bool ok = mbar_wait(&bar[s], (uint32_t)((i / ST) & 1), err, 2);
         if (!__syncthreads_and(ok)) {
             // a load never completed: wait (bounded) for the copies still in flight, leave a NaN
             if (tid == 0) {
                 for (int j = i; j < my_n && j <= i + ST - 1; ++j)
-                    mbar_wait(&bar[j % ST], (uint32_t)((j / ST) & 1), nullptr, 2);
+                    mbar_wait(&bar[j % ST], (uint32_t)((j / ST) & 1), err, 2);
                 part[blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
             }
             __syncthreads();
@@ -387,6 +392,11 @@ __global__ void __launch_bounds__(TmaPair<N, ST, MINB, LINES>::NT, MINB)
                 for (int j = i; j < my_n && j <= i + ST - 1; ++j)
                     mbar_wait(&bar[j % ST], (uint32_t)((j / ST) & 1), err, 2);
             __syncthreads();
+            if (MODE == 0 && !err)  // a caller's field
+                for (long q = 0; q < long(my_n - i) * L; ++q) {
+                    const long gl = ((long)blockIdx.x + (i + q / L) * (long)gridDim.x) * L + q % L;
+                    if (gl % W < VW) fill_nan(data, AXIS == 1 ? size_t(gl / W) * N * W + size_t(gl % W) : size_t(gl), S, N);
+                }
             return;
         }
         // line g holds va, line g + 1 vb: W and L are even, so both lie in one row

@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
 // The ring of P5 around one transform of direction DIR (ifdm_fft3d and the
 // slab transforms, and the adjoint's drift): the plain one-tile-per-block kernel leaves
 // nothing in flight while it transforms (256^3 complex128, one axis pass 172 us
-// against 82 us of DRAM time).
+// against 82 us of DRAM time).  err may be null: a caller's field then holds
+// NaN where a wait gave up.
 template <int N, int ST, int MINB, typename R, typename K, int DIR>
 __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
     k_fft_z_tma(cx<R> *__restrict__ data, const cx<K> *__restrict__ tw, int *__restrict__ err, int ntiles, uint32_t salt) {
@@ -264,7 +265,11 @@ __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
-        if (!ring_wait<ST>(bar, i, my_n, err)) return;
+        if (!ring_wait<ST>(bar, i, my_n, err)) {
+            for (int j = i; !err && j < my_n; ++j)
+                fill_nan(data, size_t(blockIdx.x + (long)j * gridDim.x) * L * N, 1, L * N);
+            return;
+        }
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
         const G *lp = reinterpret_cast<const G *>(slot) + l * Z::PP;
         C v[E];
@@ -316,7 +321,11 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
         for (int i = 0; i < ST - 1 && i < my_n; ++i) issue(i);
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
-        if (!ring_wait<ST>(bar, i, my_n, err)) return;
+        if (!ring_wait<ST>(bar, i, my_n, err)) {
+            for (int j = i; !err && j < my_n; ++j)
+                fill_nan(data, size_t(blockIdx.x + (long)j * gridDim.x) * L * N, 1, L * N);
+            return;
+        }
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
         const C *pa = reinterpret_cast<const C *>(slot) + (2 * lp) * Z::PP, *pb = pa + Z::PP;
         C va[E], vb[E];

@@ -240,7 +240,8 @@ void ifdm_batch_destroy(ifdm_batch *b);
  * precision == IFDM_FP64, complex64 otherwise; IFDM_MIXED computes in FP64);
  * sign -1 forward, +1 backward
  * -- the contract of the reference's fftw_mpi_plan_dft_3d plans
- * (src/CosmoBEC_MPI.cpp:176-177). */
+ * (src/CosmoBEC_MPI.cpp:176-177).  Asynchronous; lines that a device-side wait
+ * gave up on are filled with NaN (ifdm_fft_slab too). */
 int ifdm_fft3d(void *data, int n, int precision, int sign, void *stream);
 /* One axis of the local step of a slab-decomposed 3-D FFT, in place on device
  * data: the reference splits the box into x-slabs of local_n0 = n/P planes per
