@@ -19,12 +19,13 @@
 namespace ifdm {
 
 // Load one recorded step into the pass state and rebuild its drift tables;
-// conj != 0 writes the conjugate tables (the adjoint drift) instead.
+// conj != 0 writes the conjugate tables (the adjoint drift) instead.  steps < 0:
+// the step's own counter, so that its stochastic rounding repeats exactly.
 __global__ void k_replay_step(TState *__restrict__ ts, const StepLog *__restrict__ lg, int N, int conj,
                               long long steps, double2 *__restrict__ drift64, float2 *__restrict__ drift32) {
     const StepLog e = *lg;
     if (threadIdx.x == 0) {
-        ts->steps = steps;
+        ts->steps = steps < 0 ? e.steps : steps;
         ts->coefP = e.coefP;
         ts->coefQ = e.coefQ;
         ts->alpha = e.alpha;

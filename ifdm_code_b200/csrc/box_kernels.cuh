@@ -162,7 +162,6 @@ struct BoxRun {
     int win_tail;
     int timestep;          // 1: compute each step's timestep; 0: *ts holds it (one step)
     StepLog *log;          // timestep 1: append each step (may be null); 2: replay them
-    long long steps0;      // replay: step counter of the first step
     void *seg_psi, *seg_phi;  // replay: the state before each step is copied here
     // initial pass
     const void *in;        // complex128 psi in natural units, or null: psi already holds it
@@ -920,8 +919,8 @@ template <class O> struct BoxShared {
 };
 
 // Load recorded step `e` as the current one (replay of a segment).
-__device__ __forceinline__ void box_replay(TState *st, const StepLog &e, long long steps) {
-    st->steps = steps;
+__device__ __forceinline__ void box_replay(TState *st, const StepLog &e) {
+    st->steps = e.steps;
     st->coefP = e.coefP;
     st->coefQ = e.coefQ;
     st->alpha = e.alpha;
@@ -975,7 +974,7 @@ __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MI
             }
             __syncthreads();
         } else if (a.timestep == 2) {
-            if (tid == 0) box_replay(st, a.log[n], a.steps0 + n);
+            if (tid == 0) box_replay(st, a.log[n]);
             __syncthreads();
         }
         for (int p = rank; p < N; p += group) {

@@ -51,6 +51,7 @@ struct StepLog {
     double pendP, pendQ; // half kick owed after this step
     double gphase;       // accumulated dither after this step's kick
     double a, dt_KE, dt_PE, dt_QI;
+    long long steps;     // step counter of its passes (stochastic rounding)
 };
 
 }  // namespace ifdm

@@ -769,9 +769,9 @@ std::string StepEngine::share_device(bool on) {
 }
 
 // timestep: 1 each step's own (appended to log when given), 0 the one *ts_
-// holds (one step), 2 replay log[0 ..] with step counters steps0 ...; save: keep
-// the state before each step in the segment buffers.
-std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void *log, long long steps0, bool save) {
+// holds (one step), 2 replay log[0 ..]; save: keep the state before each step in
+// the segment buffers.
+std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void *log, bool save) {
     BoxRun a{};
     a.psi = psi_;
     a.phi = phi_;
@@ -793,7 +793,6 @@ std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void 
     for (int n = 0; n < nsteps; n += kMaxSteps) {
         const int cnt = std::min(kMaxSteps, nsteps - n);
         a.log = log ? (StepLog *)log + n : nullptr;
-        a.steps0 = steps0 + n;
         a.seg_psi = save ? (char *)seg_psi_ + size_t(n) * n3 * 2 * rs : nullptr;
         a.seg_phi = save ? (char *)seg_phi_ + size_t(n) * n3 * rs : nullptr;
         CUDA_TRY(box_kernels(cfg_.precision).run(cfg_.N, 0, l, a, nullptr, cnt));
@@ -986,12 +985,12 @@ std::string StepEngine::launch_passes(cudaEvent_t *ev) {
 
 std::string StepEngine::timestep_only(double dt_scale) { return launch_timestep(dt_scale); }
 std::string StepEngine::passes_only() {
-    if (box_) return box_run(1, 0, 1.0, nullptr, 0, false);
+    if (box_) return box_run(1, 0, 1.0, nullptr, false);
     return launch_passes(nullptr);
 }
 
 std::string StepEngine::step(int nsteps, double dt_scale) {
-    if (box_) return box_run(nsteps, 1, dt_scale, nullptr, 0, false);
+    if (box_) return box_run(nsteps, 1, dt_scale, nullptr, false);
     for (int i = 0; i < nsteps; ++i) {
         std::string e = launch_timestep(dt_scale);
         if (!e.empty()) return e;
@@ -1143,7 +1142,7 @@ std::string StepEngine::record(int nsteps, double dt_scale, int ckpt) {
         }
         if (box_) {  // up to the next checkpoint
             const int cnt = std::min(ckpt - n % ckpt, nsteps - n);
-            e = box_run(cnt, 1, dt_scale, lg + n, 0, false);
+            e = box_run(cnt, 1, dt_scale, lg + n, false);
             if (!e.empty()) return e;
             n += cnt - 1;
             continue;
@@ -1237,9 +1236,7 @@ std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
             CUDA_TRY(cudaMemcpyAsync((char *)seg_phi_ + size_t(n - start) * n3 * rs, phi_, n3 * rs,
                                      cudaMemcpyDeviceToDevice, stream_));
             if (n + 1 < end) {  // the last state of the segment is not needed
-                // same step counter as the forward pass, so stochastic rounding repeats exactly
-                k_replay_step<<<1, 256, 0, stream_>>>(ts_, (const StepLog *)log_ + n, cfg_.N, 0, n + 1, drift64_,
-                                                      drift32_);
+                k_replay_step<<<1, 256, 0, stream_>>>(ts_, (const StepLog *)log_ + n, cfg_.N, 0, -1, drift64_, drift32_);
                 e = launch_passes(nullptr);
                 if (!e.empty()) return e;
             }
@@ -1320,8 +1317,7 @@ std::string StepEngine::adjoint_box(const TState &fin) {
         CUDA_TRY(cudaMemcpyAsync(phi_, (char *)ckpt_phi_ + size_t(seg) * n3 * rs, n3 * rs, cudaMemcpyDeviceToDevice,
                                  stream_));
         if (end - start > 1) {
-            // same step counters as the forward pass, so stochastic rounding repeats exactly
-            std::string e = box_run(end - start - 1, 2, 1.0, (StepLog *)log_ + start, start + 1, true);
+            std::string e = box_run(end - start - 1, 2, 1.0, (StepLog *)log_ + start, true);
             if (!e.empty()) return e;
         }
         a.start = start;

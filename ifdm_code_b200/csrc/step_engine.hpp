@@ -133,7 +133,7 @@ class StepEngine {
     int box_group_ = 0;        // CTAs of the group that runs this box
     void *box_scr_ = nullptr;  // BoxScratch
     std::string init_box();
-    std::string box_run(int nsteps, int timestep, double dt_scale, void *log, long long steps0, bool save);
+    std::string box_run(int nsteps, int timestep, double dt_scale, void *log, bool save);
     std::string adjoint_box(const TState &fin);
     std::string adjoint_finish(double *g0_dev, double lambda);
     void *log_ = nullptr;  // StepLog[log_cap_]

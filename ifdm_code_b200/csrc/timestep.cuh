@@ -218,6 +218,7 @@ __device__ __forceinline__ void log_step(const TState *ts, StepLog *lg) {
     e.dt_KE = ts->dt_KE;
     e.dt_PE = ts->dt_PE;
     e.dt_QI = ts->dt_QI;
+    e.steps = ts->steps;
     *lg = e;
 }
 
