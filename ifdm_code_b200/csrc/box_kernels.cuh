@@ -163,9 +163,7 @@ struct BoxRun {
     int timestep;          // 1: compute each step's timestep; 0: *ts holds it (one step)
     StepLog *log;          // timestep 1: append each step (may be null); 2: replay them
     void *seg_psi, *seg_phi;  // replay: the state before each step is copied here
-    // initial pass
-    const void *in;        // complex128 psi in natural units, or null: psi already holds it
-    double invS, a0;
+    double a0;             // initial pass: scale factor
 };
 
 // Backward sweep over the recorded steps start .. end-1.
@@ -827,25 +825,16 @@ template <typename R_, typename K_, int N, int V> struct BoxOps {
             }
     }
 
-    // initial pass of plane p: psi in storage units and its sums
+    // initial pass: the sums of plane p
     __device__ __forceinline__ static void initial_sums(const BoxRun &a, int p) {
         const Lane q(N);
         const int l = q.l, t = q.t, tid = threadIdx.x;
-        G *psi = (G *)a.psi;
-        const double2 *in = (const double2 *)a.in;
+        const G *psi = (const G *)a.psi;
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, mx = 0.0;
         if (q.act) {
 #pragma unroll
             for (int i = 0; i < E; ++i) {
-                const size_t gi = elem(p, t, i, l);
-                G g;
-                if (in) {
-                    const double2 z = in[gi];
-                    g = mkc((R)(z.x * a.invS), (R)(z.y * a.invS));
-                    psi[gi] = g;
-                } else {
-                    g = psi[gi];
-                }
+                const G g = psi[elem(p, t, i, l)];
                 const double n2 = cnorm2(cin<double>(g));
                 s0 += (double)g.x;
                 s1 += (double)g.y;
@@ -1024,7 +1013,7 @@ __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MI
     }
 }
 
-// psi -> storage units, the initial density and potential, the state at a0
+// the initial density and potential of psi, the state at a0
 template <typename R, typename K, int N, int V>
 __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MINB)
     k_box_load(const __grid_constant__ BoxRun a, int group, int cluster) {

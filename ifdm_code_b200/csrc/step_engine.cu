@@ -845,11 +845,10 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         std::string e = reset_state(a);
         if (!e.empty()) return e;
     }
-    if (on_device && box_) {
-        // the initial pass reads psi itself
-    } else if (on_device) {
-        if (prec == 0) k_psi_in<double><<<1184, 256, 0, stream_>>>((const double2 *)psi, (double2 *)psi_, invS, n3);
-        else k_psi_in<float><<<1184, 256, 0, stream_>>>((const double2 *)psi, (float2 *)psi_, invS, n3);
+    if (on_device) {
+        const int nb = (int)std::min<size_t>(1184, (n3 + 255) / 256);
+        if (prec == 0) k_psi_in<double><<<nb, 256, 0, stream_>>>((const double2 *)psi, (double2 *)psi_, invS, n3);
+        else k_psi_in<float><<<nb, 256, 0, stream_>>>((const double2 *)psi, (float2 *)psi_, invS, n3);
 
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaEventRecord(ev_read_, stream_));
@@ -888,8 +887,6 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         a0.scr = (BoxScratch *)box_scr_;
         a0.win_rows = win_rows_;
         a0.win_tail = win_tail_;
-        a0.in = on_device ? psi : nullptr;
-        a0.invS = invS;
         a0.a0 = a;
         BoxLaunch l;
         l.group = box_group_;
@@ -897,13 +894,15 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         l.stream = stream_;
         CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
         CUDA_TRY(box_kernels(prec).load(cfg_.N, l, a0));
-        if (on_device) CUDA_TRY(cudaEventRecord(ev_read_, stream_));
     } else {
         std::string e = launch_initial_density();
         if (!e.empty()) return e;
     }
     // stream_ may still hold earlier steps: the caller's tensor is free for
-    // reuse on any stream only once the kernel that reads it has run
+    // reuse on any stream only once the kernel that reads it has run.  That is a
+    // short one of its own, so that the passes above are not waited for (24
+    // boxes set and stepped as a batch: 6.16 ms without a wait, 6.80 with one
+    // for the whole load)
     if (on_device) CUDA_TRY(cudaEventSynchronize(ev_read_));
     return "";
 }
