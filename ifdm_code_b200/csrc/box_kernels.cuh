@@ -851,21 +851,22 @@ template <typename R_, typename K_, int N, int V> struct BoxOps {
         if (tid == 0) a.scr->part[p][3] = bits_to_double(s_mx);
         __syncthreads();
     }
-    // and the half spectrum of the density less its mean, as in every later step:
-    // what is rounded to K (FP32), or to the stored half spectrum (mixed), is
-    // small where the density is near its mean, and no cell's rounding depends on
-    // another cell's density.  64^3, contrast 0.02, phi against FP64: nothing
-    // subtracted 1.6e-6 (FP32) and 2.1e-6 (mixed), the mean 2.2e-7 and 1.8e-7.
-    // The mean as a number of the storage type: the same in FP32 and mixed.
+    // and the half spectrum of the density less a constant (the k = 0 mode is
+    // dropped) near its mean: what is rounded to K (FP32), or to the stored half
+    // spectrum (mixed), is then small where the density is near its mean.  The
+    // constant is the first cell's density, held to within a factor of two of the
+    // mean so that no cell's rounding depends on a halo or a void there.  phi
+    // against FP64, 64^3, contrast 0.02: nothing subtracted 1.6e-6 (FP32) and
+    // 2.1e-6 (mixed), so 2.4e-7 and 1.9e-7, the mean itself 2.2e-7 and 1.8e-7.
     __device__ __forceinline__ static void initial_density(C *sm, SmemTw<C> tw, const BoxRun &a, const TState *st, int p) {
         const Lane q(N);
         const G *psi = (const G *)a.psi;
-        const double mu = (double)(R)st->mu;
+        const double mu = st->mu, ref = fmin(fmax(cnorm2(cin<double>(psi[0])), 0.5 * mu), 2.0 * mu);
         C w[E / 2] = {};
         if (q.act) {
             K rho[E];
 #pragma unroll
-            for (int i = 0; i < E; ++i) rho[i] = (K)(cnorm2(cin<double>(__ldcg(psi + elem(p, q.t, i, q.l)))) - mu);
+            for (int i = 0; i < E; ++i) rho[i] = (K)(cnorm2(cin<double>(psi[elem(p, q.t, i, q.l)])) - ref);
 #pragma unroll
             for (int b = 0; b < E / F0; ++b)
 #pragma unroll
