@@ -30,6 +30,7 @@
 // reductions (the same code and inputs, so the same values), which saves a barrier.
 #pragma once
 
+#include "angles.cuh"
 #include "step_kernels.cuh"
 #include "timestep.cuh"
 #include "tma.cuh"
@@ -242,19 +243,6 @@ struct GroupBarrier {
     }
 };
 
-// exp(-i p) and its pieces through sincospi: sincos(p) carries an out-of-line
-// reduction for huge arguments, and the registers saved around that call
-// (one per unrolled element) spilled kilobytes a thread.  p/pi = y + e with
-// the product's rounding error and the constant's remainder in e, which turns
-// the pair by the small angle pi e, so the argument keeps its full accuracy.
-__device__ __forceinline__ void sincos_pi(double p, double &s, double &c) {
-    const double hi = 0.31830988618379067154, lo = -1.9678676675182486e-17, pi = 3.14159265358979323846;
-    const double y = p * hi, e = pi * fma(p, lo, fma(p, hi, -y));
-    double s0, c0;
-    sincospi(y, &s0, &c0);
-    s = fma(c0, e, s0);
-    c = fma(-s0, e, c0);
-}
 // v exp(-i p) - c0, the kicked field less the offset, rounded to K once.
 template <typename K> struct BoxKick;
 template <> struct BoxKick<double> {
@@ -264,38 +252,6 @@ template <> struct BoxKick<double> {
         return cmul(v, mkc(c, -s)) - c0;
     }
 };
-// sin and cos of p to 1e-11 in FP64: the Taylor series to z^11 and z^12 on
-// |z| <= pi/4, the quadrant from 2p/pi rounded by adding 1.5 2^52; a third of
-// sincos's FP64 operations.
-__device__ __forceinline__ int sincos_quarter(double p, double &s, double &c) {
-    const double big = 6755399441055744.0;
-    const double t = p * 0.31830988618379067154, m = fma(t, 2.0, big);
-    const double z = fma(m - big, -0.5, t) * 3.14159265358979323846, z2 = z * z;
-    s = fma(z2, -1.0 / 39916800.0, 1.0 / 362880.0);
-    c = fma(z2, 1.0 / 479001600.0, -1.0 / 3628800.0);
-    s = fma(s, z2, -1.0 / 5040.0);
-    c = fma(c, z2, 1.0 / 40320.0);
-    s = fma(s, z2, 1.0 / 120.0);
-    c = fma(c, z2, -1.0 / 720.0);
-    s = fma(s, z2, -1.0 / 6.0);
-    c = fma(c, z2, 1.0 / 24.0);
-    s = fma(s * z2, z, z);
-    c = fma(c, z2, -0.5);
-    c = fma(c, z2, 1.0);
-    return __double2loint(m);  // p = z + j pi/2
-}
-template <typename K> __device__ __forceinline__ void box_sincos(double p, double &s, double &c) {
-    if constexpr (sizeof(K) == 8) {
-        sincos_pi(p, s, c);
-    } else {
-        double s0, c0;
-        const int j = sincos_quarter(p, s0, c0);
-        const double a = (j & 1) ? c0 : s0, b = (j & 1) ? -s0 : c0;
-        s = (j & 2) ? -a : a;
-        c = (j & 2) ? -b : b;
-    }
-}
-
 // FP32: the pair, its product with psi and the difference in FP64, so the
 // rounding is relative to psi - c too and nothing changes |psi| one way (an
 // FP32 pair put back on the unit circle lost 6e-9 of the norm a step).
@@ -761,7 +717,10 @@ template <typename R_, typename K_, int N, int V> struct BoxOps {
     // kick adjoint pieces at this thread's elements: theta's sine and cosine
     __device__ __forceinline__ static void kick_angle(G s, R f, double a, double b, double alpha, double &sn, double &cs) {
         const double px = (double)s.x, py = (double)s.y;
-        box_sincos<K>(a * (double)f + b * (px * px + py * py) + alpha, sn, cs);
+        const double th = a * (double)f + b * (px * px + py * py) + alpha;
+        // both to FP64's last bits; FP32, 128^3, 20 steps, replay and sweep: 3.69 ms with sincos_pi, 3.51 with the series
+        if constexpr (sizeof(K) == 8) sincos_pi(th, sn, cs);
+        else sincos_series<true>(th, sn, cs);
     }
     // w = Im(conj(g) psi exp(-i theta)), rounded as it is stored
     __device__ __forceinline__ static R adj_w(G g, G s, double sn, double cs) {
