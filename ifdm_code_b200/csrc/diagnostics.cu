@@ -137,9 +137,12 @@ __global__ void __launch_bounds__(DTile<N>::NT)
         for (int i = 0; i < 4; ++i) part[5 * size_t(blockIdx.x) + i] = o[i];
 }
 
-// out[c] = sum over blocks b (in order) of part[stride b + c], c < nv
-__global__ void k_sum_cols(const double *__restrict__ part, int nb, int stride, int nv, double *__restrict__ out) {
+// out[c] = sum over blocks b (in order) of part[stride b + c], c < nv; the error
+// bits beside them, *err_out (one copy brings back the results and the bits)
+__global__ void k_sum_cols(const double *__restrict__ part, int nb, int stride, int nv, double *__restrict__ out,
+                           const TState *__restrict__ ts, double *__restrict__ err_out) {
     __shared__ double red[32];
+    if (threadIdx.x == 0) *err_out = (double)ts->err;
     for (int c = 0; c < nv; ++c) {
         double a = 0.0;
         for (int b = threadIdx.x; b < nb; b += blockDim.x) a += part[size_t(stride) * b + c];
@@ -216,9 +219,11 @@ __global__ void __launch_bounds__(kBinThreads)
 }
 
 // out[b * 3 + c] = sum over groups of part[(group * nb + b) * 3 + c]
-__global__ void k_bin_total(const double *__restrict__ part, int groups, int nb, double *__restrict__ out) {
+__global__ void k_bin_total(const double *__restrict__ part, int groups, int nb, double *__restrict__ out,
+                            const TState *__restrict__ ts, double *__restrict__ err_out) {
     __shared__ double red[32];
     const int b = blockIdx.x;
+    if (b == 0 && threadIdx.x == 0) *err_out = (double)ts->err;
     for (int c = 0; c < 3; ++c) {
         double s = 0.0;
         for (int g = threadIdx.x; g < groups; g += blockDim.x) s += part[(size_t(g) * nb + b) * 3 + c];
@@ -271,7 +276,7 @@ std::string field_means(const EngineView &v, double S, double2 *field, double *w
         auto go = [&](auto kern, const auto *psi, const auto *phi) -> std::string {
             DG_TRY(big_smem(kern, TL::SMEM));
             kern<<<blocks, TL::NT, TL::SMEM, s>>>(psi, phi, v.ts, field, work, (const double2 *)tw);
-            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 5, 4, tot);
+            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 5, 4, tot, v.ts, tot + 6);
             DG_TRY(cudaGetLastError());
             return "";
         };
@@ -281,15 +286,13 @@ std::string field_means(const EngineView &v, double S, double2 *field, double *w
     for (int axis = 1; e.empty() && axis >= 0; --axis) {
         int np = 0;
         e = axis_k2(field, N, axis, work + off_axis(N), &np, &v.ts->err, s);
-        if (e.empty()) k_sum_cols<<<1, 1024, 0, s>>>(work + off_axis(N), np, 1, 1, tot + 4 + axis);
+        if (e.empty()) k_sum_cols<<<1, 1024, 0, s>>>(work + off_axis(N), np, 1, 1, tot + 4 + axis, v.ts, tot + 6);
     }
     if (!e.empty()) return e;
-    double h[6];
-    int err = 0;
+    double h[7];
     DG_TRY(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, s));
-    DG_TRY(cudaMemcpyAsync(&err, &v.ts->err, sizeof(err), cudaMemcpyDeviceToHost, s));
     DG_TRY(cudaStreamSynchronize(s));
-    if (err & 2) return kGaveUp;
+    if ((int)h[6] & 2) return kGaveUp;
     const double S2 = S * S, kf = 3.14159265358979323846 / xmax;  // k = pi kappa / xmax
     out[0] = h[0] / n3 * S2;
     // Parseval per axis: sum_x |d psi/dz|^2 = sum over lines of sum_k k^2 |.|^2 / N
@@ -328,7 +331,7 @@ std::string power_spectrum(const EngineView &v, double S, double2 *field, double
         auto go = [&](auto kern, const auto *psi) -> std::string {
             DG_TRY(big_smem(kern, TL::SMEM));
             kern<<<blocks, TL::NT, TL::SMEM, s>>>(psi, field, work, (const double2 *)tw, (const double2 *)twh);
-            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 1, 1, tot + 3 * kMaxBins);
+            k_sum_cols<<<1, 1024, 0, s>>>(work, blocks, 1, 1, tot + 3 * kMaxBins, v.ts, tot + 3 * kMaxBins + 1);
             DG_TRY(cudaGetLastError());
             return "";
         };
@@ -339,14 +342,12 @@ std::string power_spectrum(const EngineView &v, double S, double2 *field, double
     if (e.empty()) e = fft_half_axis(field, N, 0, v.ts, s);
     if (!e.empty()) return e;
     k_bin_half<<<kBinBlocks, kBinThreads, 0, s>>>(field, N, half_pitch<double>(N), nbins, ed, work + off_bins(N));
-    k_bin_total<<<nbins, 256, 0, s>>>(work + off_bins(N), kBinBlocks, nbins, tot);
+    k_bin_total<<<nbins, 256, 0, s>>>(work + off_bins(N), kBinBlocks, nbins, tot, v.ts, tot + 3 * kMaxBins + 1);
     DG_TRY(cudaGetLastError());
-    std::vector<double> h(3 * kMaxBins + 1);
-    int err = 0;
+    std::vector<double> h(3 * kMaxBins + 2);
     DG_TRY(cudaMemcpyAsync(h.data(), tot, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s));
-    DG_TRY(cudaMemcpyAsync(&err, &v.ts->err, sizeof(err), cudaMemcpyDeviceToHost, s));
     DG_TRY(cudaStreamSynchronize(s));
-    if (err & 2) return kGaveUp;
+    if ((int)h[3 * kMaxBins + 1] & 2) return kGaveUp;
     const double mean = h[3 * kMaxBins] / n3;
     if (mean_rho) *mean_rho = mean * S * S;
     // delta_k = rho_k / mean for kappa != 0 (the bins exclude kappa = 0)

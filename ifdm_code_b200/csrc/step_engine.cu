@@ -155,13 +155,16 @@ template <typename R_, typename K_, int N> struct Box {
             CUDA_TRY(prep(k_yx_tma<R, K, N, 1, 0, +1>, TT::SMEM));
             CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 1, 0>, TX::SMEM));
             CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 2, 0>, TX::SMEM));
-            if constexpr (kFftTma) {
+            if constexpr (kFftTma && !kPair) {  // the callers' fields (axis_pass)
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 1, 0, -1, true>, TT::SMEM));
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 1, 0, +1, true>, TT::SMEM));
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, -1, true>, TX::SMEM));
+                CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, +1, true>, TX::SMEM));
+            }
+            if constexpr (kFftTma && std::is_same<R, double>::value) {  // the diagnostics
                 CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, -1>, TX::SMEM));
-                CUDA_TRY(prep(k_yx_tma<R, K, N, 2, 0, +1>, TX::SMEM));
-                if constexpr (std::is_same<R, double>::value) {
-                    CUDA_TRY(prep(k_line_k2_tma<N, 1>, TT::SMEM));
-                    CUDA_TRY(prep(k_line_k2_tma<N, 2>, TX::SMEM));
-                }
+                CUDA_TRY(prep(k_line_k2_tma<N, 1>, TT::SMEM));
+                CUDA_TRY(prep(k_line_k2_tma<N, 2>, TX::SMEM));
             }
             // persistent grids: every block resident at once (one wave)
             int by = 0, bx = 0;
@@ -174,10 +177,12 @@ template <typename R_, typename K_, int N> struct Box {
                 CUDA_TRY(prep(k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY>, TPY::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 1, 0, PSTX, PBX>, TPX::SMEM));
                 CUDA_TRY(prep(k_yx_tma_pair<N, 2, 2, 0, PSTX, PBX>, TPX::SMEM));
-                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF>, TPF::SMEM));
-                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF>, TPF::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY, 8, true>, TPY::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY, 8, true>, TPY::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF, true>, TPF::SMEM));
+                CUDA_TRY(prep(k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF, true>, TPF::SMEM));
                 int pf = 0;
-                CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF>,
+                CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF, true>,
                                                                        TPF::NT, TPF::SMEM));
                 pfgrid = sms * (pf > 0 ? pf : 1);
                 int py = 0, px = 0;
@@ -473,20 +478,20 @@ template <typename R_, typename K_, int N> struct Box {
             if constexpr (kPair) {
                 const int nt = int(lines / (axis == 1 ? TPY::L : TPF::L));
                 if (axis == 1) {
-                    if (sign < 0) k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
-                    else k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
+                    if (sign < 0) k_yx_tma_pair<N, 1, 0, -1, PSTY, PBY, 8, true><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
+                    else k_yx_tma_pair<N, 1, 0, +1, PSTY, PBY, 8, true><<<pygrid, TPY::NT, TPY::SMEM, s>>>(m, data, N, N, nt, nullptr, nullptr, tw);
                 } else {
-                    if (sign < 0) k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
-                    else k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                    if (sign < 0) k_yx_tma_pair<N, 2, 0, -1, PSTX, PBF, PLF, true><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
+                    else k_yx_tma_pair<N, 2, 0, +1, PSTX, PBF, PLF, true><<<pfgrid, TPF::NT, TPF::SMEM, s>>>(m, data, planes, planes, nt, nullptr, nullptr, tw);
                 }
             } else if (axis == 1) {
                 const int nt = int(lines / TT::L);
-                if (sign < 0) k_yx_tma<R, K, N, 1, 0, -1><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
-                else k_yx_tma<R, K, N, 1, 0, +1><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
+                if (sign < 0) k_yx_tma<R, K, N, 1, 0, -1, true><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
+                else k_yx_tma<R, K, N, 1, 0, +1, true><<<ygrid, TT::NT, TT::SMEM, s>>>(m, data, N, N, nt, nullptr, 2, nullptr, tw);
             } else {
                 const int nt = int(lines / TX::L);
-                if (sign < 0) k_yx_tma<R, K, N, 2, 0, -1><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
-                else k_yx_tma<R, K, N, 2, 0, +1><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
+                if (sign < 0) k_yx_tma<R, K, N, 2, 0, -1, true><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
+                else k_yx_tma<R, K, N, 2, 0, +1, true><<<xgrid, TX::NT, TX::SMEM, s>>>(m, data, planes, planes, nt, nullptr, 3, nullptr, tw);
             }
             return "";
         }

@@ -140,6 +140,24 @@ __device__ __forceinline__ uint32_t pass_salt(const TState *ts, int pass) {
     return mix32((uint32_t)ts->steps * 16u + (uint32_t)pass);
 }
 
+// A transform of a caller's field has no error word: NaN into this block's
+// tiles (L lines of N elements each) from its i-th on, which a wait gave up.
+// Lines along y (AXIS 1) or x (2; W and VW as in the axis passes), or rows (3).
+template <int AXIS, typename G>
+__device__ __noinline__ void give_up_lines(G *data, int N, int W, int VW, int L, int ntiles, int i) {
+    const float q = __int_as_float(0x7fffffff);
+    G v;
+    v.x = q;
+    v.y = q;
+    const size_t S = AXIS == 3 ? 1 : AXIS == 1 ? size_t(W) : size_t(N) * W;
+    for (long tile = (long)blockIdx.x + (long)i * gridDim.x; tile < ntiles; tile += gridDim.x)
+        for (int f = threadIdx.x; f < L * N; f += blockDim.x) {
+            const long g = tile * L + f % L;
+            const size_t b = AXIS == 3 ? size_t(g) * N : AXIS == 1 ? size_t(g / W) * N * W + size_t(g % W) : size_t(g);
+            if (AXIS == 3 || g % W < VW) data[b + (f / L) * S] = v;
+        }
+}
+
 // Deterministic block sum of three doubles; thread 0 writes out[0..2].
 __device__ __forceinline__ void block_sum3(double a, double b, double c, double *out) {
     __shared__ double red[3][32];

@@ -65,17 +65,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
     return false;
 }
 
-// NaN into elements first, first + stride, ... (count of them) of a field of
-// complex numbers, all threads of the block: the lines a kernel without an
-// error word gave up
-template <typename G> __device__ __noinline__ void fill_nan(G *data, size_t first, size_t stride, int count) {
-    const float q = __int_as_float(0x7fffffff);
-    G v;
-    v.x = q;
-    v.y = q;
-    for (int n = threadIdx.x; n < count; n += blockDim.x) data[first + n * stride] = v;
-}
-
 // generic-proxy accesses to shared memory before later async-proxy writes
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -266,8 +266,7 @@ __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, err)) {
-            for (int j = i; !err && j < my_n; ++j)
-                fill_nan(data, size_t(blockIdx.x + (long)j * gridDim.x) * L * N, 1, L * N);
+            if (!err) give_up_lines<3>(data, N, 1, 1, L, ntiles, i);
             return;
         }
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;
@@ -322,8 +321,7 @@ __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
     for (int i = 0; i < my_n; ++i) {
         if (tid == 0 && i + ST - 1 < my_n) issue(i + ST - 1);
         if (!ring_wait<ST>(bar, i, my_n, err)) {
-            for (int j = i; !err && j < my_n; ++j)
-                fill_nan(data, size_t(blockIdx.x + (long)j * gridDim.x) * L * N, 1, L * N);
+            if (!err) give_up_lines<3>(data, N, 1, 1, L, ntiles, i);
             return;
         }
         unsigned char *slot = smraw + size_t(i % ST) * Z::SLOT5;

@@ -140,13 +140,15 @@ int main() {
         constexpr int A = decltype(axis)::value;
         using T = TmaTile<double, double, N, A>;
         auto k = big(k_yx_tma<double, double, N, A, 0, -1>, T::SMEM);
+        auto kf = big(k_yx_tma<double, double, N, A, 0, -1, true>, T::SMEM);
         check<double>(A == 1 ? "y-fp64" : "x-fp64", T::L, A == 1 ? 1 : 0, ts, [&](double2 *d, TState *t) {
-            k<<<3, T::NT, T::SMEM>>>(field_map(d, true, A, T::L), d, A == 1 ? N : 1, A == 1 ? N : 1, N / T::L, t, 2, nullptr, w64);
+            (t ? k : kf)<<<3, T::NT, T::SMEM>>>(field_map(d, true, A, T::L), d, A == 1 ? N : 1, A == 1 ? N : 1, N / T::L, t, 2, nullptr, w64);
         });
         using P = TmaPair<N, 2, 3>;
         auto kp = big(k_yx_tma_pair<N, A, 0, -1, 2, 3>, P::SMEM);
+        auto kpf = big(k_yx_tma_pair<N, A, 0, -1, 2, 3, 8, true>, P::SMEM);
         check<float>(A == 1 ? "y-fp32" : "x-fp32", P::L, A == 1 ? 1 : 0, ts, [&](float2 *d, TState *t) {
-            kp<<<3, P::NT, P::SMEM>>>(field_map(d, false, A, P::L), d, A == 1 ? N : 1, A == 1 ? N : 1, N / P::L, t, nullptr, w32);
+            (t ? kp : kpf)<<<3, P::NT, P::SMEM>>>(field_map(d, false, A, P::L), d, A == 1 ? N : 1, A == 1 ? N : 1, N / P::L, t, nullptr, w32);
         });
     };
     plain(std::integral_constant<int, 1>{});
