@@ -230,7 +230,9 @@ std::string BatchEngine::capture_body(int nsteps) {
             l.boxes = nb;
             l.cluster = true;
             l.stream = c.side;
-            CUDA_TRY(box_kernels(precision_).run(c.N, V, l, BoxRun{}, (const BoxRun *)c.d_boxes, nsteps));
+            for (int n = 0; n < nsteps; n += kBoxLaunchSteps)
+                CUDA_TRY(box_kernels(precision_).run(c.N, V, l, BoxRun{}, (const BoxRun *)c.d_boxes,
+                                                     std::min(kBoxLaunchSteps, nsteps - n)));
         } else if (c.box) {
             for (int s = 0; s < nsteps; ++s)
                 for (int p = 0; p < kBoxPhases; ++p)

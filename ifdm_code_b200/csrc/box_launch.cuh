@@ -10,6 +10,8 @@
 
 namespace ifdm {
 
+constexpr int kBoxLaunchSteps = 512;  // most steps per launch (tens of milliseconds at 128^3)
+
 // `boxes` groups of `group` CTAs each; a group is a cluster or (one box) the
 // whole grid of a cooperative launch.
 struct BoxLaunch {

@@ -794,9 +794,8 @@ std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void 
     l.cluster = box_cluster_;
     l.stream = stream_;
     const size_t n3 = n3_(), rs = storage_bytes(cfg_.precision);
-    constexpr int kMaxSteps = 512;  // steps per launch (tens of milliseconds at 128^3)
-    for (int n = 0; n < nsteps; n += kMaxSteps) {
-        const int cnt = std::min(kMaxSteps, nsteps - n);
+    for (int n = 0; n < nsteps; n += kBoxLaunchSteps) {
+        const int cnt = std::min(kBoxLaunchSteps, nsteps - n);
         a.log = log ? (StepLog *)log + n : nullptr;
         a.seg_psi = save ? (char *)seg_psi_ + size_t(n) * n3 * 2 * rs : nullptr;
         a.seg_phi = save ? (char *)seg_phi_ + size_t(n) * n3 * rs : nullptr;

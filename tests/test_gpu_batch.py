@@ -185,3 +185,21 @@ def test_batch_steps_of_other_sizes_queued_behind_each_other(mode):
         assert np.array_equal(x, y)
     for s in sims:
         s.close()
+
+
+def test_batch_longer_than_one_launch():
+    # clusters run at most 512 steps a launch; the next launch carries on
+    sims, psis, _ = _boxes("fp64", [16, 32, 16])
+    with ifdm.Batch(sims) as b:
+        b.step(1030, [1e-4] * 3)
+        b.synchronize()
+        got = [(s.get_psi(), s.state()["steps"]) for s in sims]
+        for s, p in zip(sims, psis):
+            s.set_psi(p, A0)
+        for n in (512, 512, 6):
+            b.step(n, [1e-4] * 3)
+        b.synchronize()
+        for s, (psi, steps) in zip(sims, got):
+            assert steps == s.state()["steps"] == 1030 and np.array_equal(s.get_psi(), psi)
+    for s in sims:
+        s.close()
