@@ -147,7 +147,8 @@ template <int DIR> struct Bfly<16, DIR> {
 // ------------------------------------------------------------- arguments ---
 // Words the CTAs of a group share in global memory.
 struct BoxScratch {
-    unsigned long long ctr;       // barrier arrivals (a multiple of the group size between launches)
+    unsigned long long ctr[2];    // barrier arrivals of groups of N and of N/2 CTAs (a multiple of the
+                                  // group's size between launches)
     unsigned long long mx[2][2];  // max |phi|, max |psi|^2 of the previous step, by step parity
     double cnext[2];              // mean of the kicked field (the next offset c)
     double part[128][4];          // initial pass: sums of psi, |psi|^2 and max |psi|^2 per plane
@@ -896,7 +897,7 @@ __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MI
     gk_fill(s.gk);
     if (tid == 0) *st = *a.ts;
     GroupBarrier bar;
-    bar.init(&a.scr->ctr, group, cluster != 0, &a.ts->err, &s.tail->ok);
+    bar.init(&a.scr->ctr[group != N], group, cluster != 0, &a.ts->err, &s.tail->ok);
     __syncthreads();
     G *psi = (G *)a.psi, *rhok = (G *)a.rhok;
     R *phi = (R *)a.phi;
@@ -988,7 +989,7 @@ __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MI
         st->a = a.a0;
     }
     GroupBarrier bar;
-    bar.init(&a.scr->ctr, group, cluster != 0, &a.ts->err, &s.tail->ok);
+    bar.init(&a.scr->ctr[group != N], group, cluster != 0, &a.ts->err, &s.tail->ok);
     __syncthreads();
     G *rhok = (G *)a.rhok;
     for (int p = rank; p < N; p += group) O::initial_sums(a, p);
@@ -1034,7 +1035,7 @@ __global__ void __launch_bounds__(BoxOps<R, K, N, V>::NT, BoxOps<R, K, N, V>::MI
     BoxShared<O> s(smraw, a.tw);
     TState *st = &s.tail->st;
     GroupBarrier bar;
-    bar.init(&a.scr->ctr, group, cluster != 0, a.err, &s.tail->ok);
+    bar.init(&a.scr->ctr[group != N], group, cluster != 0, a.err, &s.tail->ok);
     __syncthreads();
     G *g = (G *)a.g, *rhok = (G *)a.rhok;
     const size_t n3 = size_t(N) * N * N;

@@ -639,6 +639,7 @@ const BoxKernels &box_kernels(int precision) {
 
 // ------------------------------------------------------------ StepEngine --
 StepEngine::~StepEngine() {
+    leave_full_boxes();
     cudaFree(box_scr_);
     cudaFree(psi_);
     cudaFree(phi_);
@@ -752,24 +753,79 @@ std::string StepEngine::init_box() {
         }
         resident = it->second;
     }
-    box_half_ = resident == 1 && !box_cluster_;
+    int sms = 0;
+    CUDA_TRY(cudaGetDevice(&dev_));
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_));
+    box_half_ = resident == 1 && !box_cluster_ && sms / (N / 2) >= 3;
     box_ = resident >= 1 && std::getenv("IFDM_NO_FUSE") == nullptr;
+    if (box_ && box_half_) {
+        std::string e = join_full_boxes();
+        if (!e.empty()) return e;
+    }
+    box_half_ = box_half_ && box_;
     CUDA_TRY(cudaMalloc(&box_scr_, sizeof(BoxScratch)));
     CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
     return "";
 }
 
-// Several boxes of this size step at the same time.  Where the device holds one
-// group of N CTAs (96^3, FP32 128^3: a CTA an SM), the boxes would take turns
-// and 52 of 148 SMs idle: groups of N/2 with two planes a CTA let two or three
-// boxes run side by side, which costs one box time (a step's phases double, its
-// barriers do not), so only then.  The results do not depend on the group.
-std::string StepEngine::share_device(bool on) {
-    const int group = on && box_half_ ? cfg_.N / 2 : cfg_.N;
-    if (!box_ || group == box_group_) return "";
-    // the barrier's counter is a multiple of the group when a launch starts
-    CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
-    box_group_ = group;
+// Boxes of 96^3 hold a CTA on each of 96 SMs, so a second group does not fit
+// beside one and the boxes would take turns with 52 of 148 SMs idle.  Groups of
+// N/2 with two planes a CTA let three boxes run side by side, which costs one box
+// time (a step's phases double, its barriers do not): taken while a batch works
+// on several, or while another such box has work in flight.  One step of four
+// contexts stepped in turn, us, whole / half groups: FP32 218 / 127, mixed 320 /
+// 199, FP64 290 / 224 (a launch per pass: 182, 285, 297).  FP32 128^3 keeps whole
+// groups: two halves of it gain nothing (329 / 336).  The results do not depend
+// on the group.
+namespace {
+struct FullBoxes {
+    std::mutex m;
+    std::vector<StepEngine *> all;
+};
+FullBoxes &full_boxes() {
+    static FullBoxes f;
+    return f;
+}
+}  // namespace
+
+std::string StepEngine::join_full_boxes() {
+    CUDA_TRY(cudaEventCreateWithFlags(&ev_run_, cudaEventDisableTiming));
+    std::lock_guard<std::mutex> lk(full_boxes().m);
+    full_boxes().all.push_back(this);
+    return "";
+}
+void StepEngine::leave_full_boxes() {
+    if (!ev_run_) return;
+    {
+        std::lock_guard<std::mutex> lk(full_boxes().m);
+        auto &v = full_boxes().all;
+        v.erase(std::remove(v.begin(), v.end(), this), v.end());
+    }
+    cudaEventDestroy(ev_run_);
+}
+void StepEngine::pick_group() {
+    if (!box_half_) return;
+    bool other = shared_;
+    if (!other) {
+        // a query is refused while another thread captures a graph, unless in relaxed mode
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        {
+            std::lock_guard<std::mutex> lk(full_boxes().m);
+            for (StepEngine *o : full_boxes().all) {
+                if (o == this || o->dev_ != dev_) continue;
+                const cudaError_t e = cudaEventQuery(o->ev_run_);
+                other = e == cudaErrorNotReady;
+                if (e != cudaSuccess) cudaGetLastError();
+                if (other) break;
+            }
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    box_group_ = other ? cfg_.N / 2 : cfg_.N;
+}
+std::string StepEngine::mark_run() {
+    if (box_half_) CUDA_TRY(cudaEventRecord(ev_run_, stream_));
     return "";
 }
 
@@ -988,12 +1044,18 @@ std::string StepEngine::launch_passes(cudaEvent_t *ev) {
 
 std::string StepEngine::timestep_only(double dt_scale) { return launch_timestep(dt_scale); }
 std::string StepEngine::passes_only() {
-    if (box_) return box_run(1, 0, 1.0, nullptr, false);
-    return launch_passes(nullptr);
+    if (!box_) return launch_passes(nullptr);
+    pick_group();
+    std::string e = box_run(1, 0, 1.0, nullptr, false);
+    return e.empty() ? mark_run() : e;
 }
 
 std::string StepEngine::step(int nsteps, double dt_scale) {
-    if (box_) return box_run(nsteps, 1, dt_scale, nullptr, false);
+    if (box_) {
+        pick_group();
+        std::string e = box_run(nsteps, 1, dt_scale, nullptr, false);
+        return e.empty() ? mark_run() : e;
+    }
     for (int i = 0; i < nsteps; ++i) {
         std::string e = launch_timestep(dt_scale);
         if (!e.empty()) return e;
@@ -1137,6 +1199,7 @@ std::string StepEngine::record(int nsteps, double dt_scale, int ckpt) {
     ckpt_every_ = ckpt;
     recorded_ = 0;
     StepLog *lg = static_cast<StepLog *>(log_);
+    pick_group();
     for (int n = 0; n < nsteps; ++n) {
         if (n % ckpt == 0) {
             const size_t k = size_t(n / ckpt);
@@ -1157,7 +1220,7 @@ std::string StepEngine::record(int nsteps, double dt_scale, int ckpt) {
         if (!e.empty()) return e;
     }
     recorded_ = nsteps;
-    return "";
+    return mark_run();
 }
 
 // one kick adjoint on g_: w, pw = phi_s[w], combine
@@ -1219,7 +1282,9 @@ std::string StepEngine::adjoint(const double *g_final_dev, double *g0_dev) {
         k_scale_in<float><<<1184, 256, 0, stream_>>>((const double2 *)g_final_dev, (float2 *)g_, S_ * lambda, n3);
     CUDA_TRY(cudaGetLastError());
     if (box_) {
+        pick_group();
         std::string eb = adjoint_box(fin);
+        if (eb.empty()) eb = mark_run();
         if (!eb.empty()) return eb;
         return adjoint_finish(g0_dev, lambda);
     }

@@ -70,7 +70,7 @@ class StepEngine {
     // Adjoint support.  record(): nsteps fixed-mode steps that keep a per-step
     // log of the coefficients and a checkpoint of (psi, phi) every ckpt steps.
     std::string record(int nsteps, double dt_scale, int ckpt);
-    std::string share_device(bool on);  // other boxes of this size run at the same time
+    void share_device(bool on) { shared_ = on; }  // other boxes of this size run at the same time
     // gradient of a real loss through the recorded steps: g_final = dL/dpsi_final
     // (complex128, natural units, dL/dRe + i dL/dIm) -> g0 = dL/dpsi_0; both
     // device pointers.  Leaves the context's state at an intermediate step.
@@ -129,8 +129,15 @@ class StepEngine {
     // adjoint buffers
     // one-launch box kernels (box_kernels.cuh): N <= 128 where a plane fits
     bool box_ = false, box_cluster_ = false;
-    bool box_half_ = false;    // one group of N CTAs fills the device (share_device)
+    bool box_half_ = false;    // one group of N CTAs fills the device (pick_group)
+    bool shared_ = false;
     int box_group_ = 0;        // CTAs of the group that runs this box
+    int dev_ = 0;
+    cudaEvent_t ev_run_ = nullptr;  // box_half_: after this box's latest run
+    std::string join_full_boxes();
+    void leave_full_boxes();
+    void pick_group();
+    std::string mark_run();
     void *box_scr_ = nullptr;  // BoxScratch
     std::string init_box();
     std::string box_run(int nsteps, int timestep, double dt_scale, void *log, bool save);

@@ -153,3 +153,29 @@ def test_batch_record_in_half_groups(prec, n):
         s.step(5, 0.01)  # whole groups again
         assert s.state()["device_error"] == 0 and np.array_equal(s.get_psi(), want[i][0]), i
         s.close()
+
+
+@pytest.mark.parametrize("prec,n", [("fp32", 96), ("fp64", 96), ("mixed", 96), ("fp32", 128)])
+def test_full_boxes_side_by_side(prec, n):
+    # boxes of a CTA an SM take half groups while another one has work in
+    # flight, whole ones alone: the same bits, with the group changing between
+    # the calls of one box
+    psis = [zeldovich_psi(n, seed=n + i) for i in range(4)]
+    want = []
+    for p in psis:
+        with ifdm.Simulation(MFDM, 0.0, XMAX, n, precision=prec) as s:
+            s.set_psi(p, A0)
+            s.step(24, 0.01)
+            want.append((s.get_psi(), s.get_phi()))
+    sims = [ifdm.Simulation(MFDM, 0.0, XMAX, n, precision=prec) for _ in psis]
+    for s, p in zip(sims, psis):
+        s.set_psi(p, A0)
+    for _ in range(5):
+        for s in sims:
+            s.step(4, 0.01)
+    for s, w in zip(sims, want):
+        s.synchronize()
+        s.step(4, 0.01)
+        assert s.state()["device_error"] == 0
+        assert np.array_equal(s.get_psi(), w[0]) and np.array_equal(s.get_phi(), w[1])
+        s.close()
