@@ -97,7 +97,7 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
         CUDA_TRY(cudaEventCreateWithFlags(&c.join, cudaEventDisableTiming));
         for (int v = 0; v < 2; ++v) {
             int fit = 0;
-            std::string e = c.box ? K_->box_setup(c.N, v) : K_->setup(c.N, v, c.smem, &fit);
+            std::string e = c.box ? K_->box_setup(c.N, v) : K_->setup(c.N, c.smem, &fit);
             if (e.empty() && c.box) e = bk.setup(c.N, v);
             if (!e.empty()) return e;
         }
@@ -177,7 +177,6 @@ std::string BatchEngine::prepare(const double *dt_scale) {
     for (size_t ci = 0; ci < cls_.size(); ++ci) {
         Class &c = cls_[ci];
         const int nb = (int)c.boxes.size();
-        const int V = knobs.plan[batch_size_index(c.N)] ? 1 : 0;
         // on the batch's own stream: an earlier step still in flight reads these
         // tables, and the next launch must not run before they have landed
         CUDA_TRY(cudaMemcpyAsync(c.d_boxes, hb[ci].data(), hb[ci].size(), cudaMemcpyHostToDevice, stream_));
@@ -187,7 +186,7 @@ std::string BatchEngine::prepare(const double *dt_scale) {
             for (int p = 0; p < kBoxPhases; ++p) c.step_items += (long long)c.items[p] * nb;
             continue;
         }
-        std::string e = K_->setup(c.N, V, c.smem, &c.fit);
+        std::string e = K_->setup(c.N, c.smem, &c.fit);
         if (!e.empty()) return e;
         if (c.fit < 1) return "batch: the batch kernel does not fit on an SM";
         const double share = double(nb) * c.N * c.N * c.N / work_all;
@@ -248,11 +247,11 @@ std::string BatchEngine::capture_body(int nsteps) {
             a.next = c.d_ctr;
             a.done = c.d_ctr + 1;
             a.status = d_status_;
-            CUDA_TRY(K_->persistent(c.N, V, c.grid, c.smem, c.side, a));
+            CUDA_TRY(K_->persistent(c.N, c.grid, c.smem, c.side, a));
         } else {
             for (int s = 0; s < nsteps; ++s)
                 for (int p = 0; p < kBatchPhases; ++p)
-                    CUDA_TRY(K_->phase(c.N, V, p, c.items[p], nb, c.smem, c.side, (const BatchBox *)c.d_boxes));
+                    CUDA_TRY(K_->phase(c.N, p, c.items[p], nb, c.smem, c.side, (const BatchBox *)c.d_boxes));
         }
         CUDA_TRY(cudaEventRecord(c.join, c.side));
         CUDA_TRY(cudaStreamWaitEvent(stream_, c.join, 0));
@@ -394,21 +393,25 @@ std::string BatchEngine::tune(int trial_steps, const double *dt_scale, double *b
             }
             return "";
         };
-        // 1) schedule: persistent kernels, or one launch per phase
-        {
+        // only what changes a launch of this batch: the schedule where a size has two,
+        // the persistent shapes where boxes are tiled
+        const bool tiled = std::any_of(cls_.begin(), cls_.end(), [](const Class &c) { return !c.box; });
+        const bool two = tiled || std::any_of(cls_.begin(), cls_.end(), [](const Class &c) { return c.group > 0; });
+        // 1) schedule: one kernel for all steps, or one launch per phase
+        if (two) {
             BatchKnobs k = best;
             k.mode = 1 - k.mode;
             err = consider(k);
         }
         // 2) persistent shape: CTAs per SM, then the group size of the item order
-        for (int bps = 1; bps <= 4 && err.empty(); ++bps) {
+        for (int bps = 1; bps <= 4 && tiled && err.empty(); ++bps) {
             BatchKnobs k = best;
             k.mode = 0;
             k.blocks_per_sm = bps;
             err = consider(k);
         }
         const int cand[3] = {(n + 1) / 2, (n + 3) / 4, 8};
-        for (int ci = 0; ci < 3 && err.empty(); ++ci) {
+        for (int ci = 0; ci < 3 && tiled && err.empty(); ++ci) {
             if (best.mode != 0 || cand[ci] >= n) continue;
             BatchKnobs k = best;
             k.group = cand[ci];

@@ -353,9 +353,9 @@ template <typename R, typename K, int N, class P> struct BatchOps {
     }
 };
 
-// One persistent kernel per (precision, grid size, radix plan): every box of
+// One persistent kernel per (precision, grid size): every box of
 // the launch has size N.  Launches of different sizes run side by side.
-template <typename R, typename K, int N, int V>
+template <typename R, typename K, int N>
 __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
     using Ops = BatchOps<R, K, N, Plan<N>>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
 // size (blockIdx.y = box, blockIdx.x = tile): the other batch schedule, a
 // CUDA graph of such launches, which the autotuner weighs against the
 // persistent kernel.
-template <typename R, typename K, int N, int V, int PH>
+template <typename R, typename K, int N, int PH>
 __global__ void __launch_bounds__(kBatchThreads) k_batch_phase(const BatchBox *boxes) {
     extern __shared__ __align__(16) unsigned char smraw[];
     BatchOps<R, K, N, Plan<N>>::template phase<PH>(smraw, boxes[blockIdx.y], (int)blockIdx.x);

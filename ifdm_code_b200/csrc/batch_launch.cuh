@@ -15,12 +15,11 @@ namespace ifdm {
 struct BatchKernels {
     // items per phase and dynamic shared memory of an N-box; false if N is not a batch size
     bool (*items)(int N, int *items, size_t *smem);
-    // set the shared-memory attributes of the (N, V) kernels; *fit = persistent CTAs per SM that fit
-    std::string (*setup)(int N, int V, size_t smem, int *fit);
-    cudaError_t (*persistent)(int N, int V, int grid, size_t smem, cudaStream_t s, const BatchArgs &a);
-    cudaError_t (*phase)(int N, int V, int ph, int tiles, int nboxes, size_t smem, cudaStream_t s,
-                         const BatchBox *boxes);
-    // the per-phase kernels of the boxes whose plane fits a CTA (box_kernels.cuh)
+    // tiled boxes: set the kernels' shared-memory attributes; *fit = persistent CTAs per SM that fit
+    std::string (*setup)(int N, size_t smem, int *fit);
+    cudaError_t (*persistent)(int N, int grid, size_t smem, cudaStream_t s, const BatchArgs &a);
+    cudaError_t (*phase)(int N, int ph, int tiles, int nboxes, size_t smem, cudaStream_t s, const BatchBox *boxes);
+    // the per-phase kernels of the boxes whose plane fits a CTA (box_kernels.cuh), radix plan V
     std::string (*box_setup)(int N, int V);
     cudaError_t (*box_phase)(int N, int V, int ph, int nboxes, cudaStream_t s, const BoxRun *boxes);
 };
@@ -28,39 +27,39 @@ constexpr int kBoxPhases = 6;  // timestep, A .. E
 
 const BatchKernels &batch_kernels(int precision);  // 0 FP64, 1 FP32, 2 mixed
 
-template <typename R, typename K, int N, int V> struct BatchLaunch {
+template <typename R, typename K, int N> struct BatchLaunch {
     static std::string setup(size_t smem, int *fit) {
         const int sm = (int)smem;
-        cudaError_t e = cudaFuncSetAttribute(k_batch<R, K, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        cudaError_t e = cudaFuncSetAttribute(k_batch<R, K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         const void *ph[kBatchPhases] = {
-            (const void *)k_batch_phase<R, K, N, V, 0>, (const void *)k_batch_phase<R, K, N, V, 1>,
-            (const void *)k_batch_phase<R, K, N, V, 2>, (const void *)k_batch_phase<R, K, N, V, 3>,
-            (const void *)k_batch_phase<R, K, N, V, 4>, (const void *)k_batch_phase<R, K, N, V, 5>,
-            (const void *)k_batch_phase<R, K, N, V, 6>, (const void *)k_batch_phase<R, K, N, V, 7>,
-            (const void *)k_batch_phase<R, K, N, V, 8>, (const void *)k_batch_phase<R, K, N, V, 9>};
+            (const void *)k_batch_phase<R, K, N, 0>, (const void *)k_batch_phase<R, K, N, 1>,
+            (const void *)k_batch_phase<R, K, N, 2>, (const void *)k_batch_phase<R, K, N, 3>,
+            (const void *)k_batch_phase<R, K, N, 4>, (const void *)k_batch_phase<R, K, N, 5>,
+            (const void *)k_batch_phase<R, K, N, 6>, (const void *)k_batch_phase<R, K, N, 7>,
+            (const void *)k_batch_phase<R, K, N, 8>, (const void *)k_batch_phase<R, K, N, 9>};
         for (int p = 0; p < kBatchPhases && e == cudaSuccess; ++p)
             e = cudaFuncSetAttribute(ph[p], cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(fit, k_batch<R, K, N, V>, kBatchThreads, smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(fit, k_batch<R, K, N>, kBatchThreads, smem);
         return e == cudaSuccess ? "" : std::string("batch kernel setup: ") + cudaGetErrorString(e);
     }
     static cudaError_t persistent(int grid, size_t smem, cudaStream_t s, const BatchArgs &a) {
-        k_batch<R, K, N, V><<<grid, kBatchThreads, smem, s>>>(a);
+        k_batch<R, K, N><<<grid, kBatchThreads, smem, s>>>(a);
         return cudaGetLastError();
     }
     static cudaError_t phase(int ph, int tiles, int nboxes, size_t smem, cudaStream_t s, const BatchBox *b) {
         const dim3 g((unsigned)tiles, (unsigned)nboxes);
         switch (ph) {
-            case 0: k_batch_phase<R, K, N, V, 0><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 1: k_batch_phase<R, K, N, V, 1><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 2: k_batch_phase<R, K, N, V, 2><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 3: k_batch_phase<R, K, N, V, 3><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 4: k_batch_phase<R, K, N, V, 4><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 5: k_batch_phase<R, K, N, V, 5><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 6: k_batch_phase<R, K, N, V, 6><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 7: k_batch_phase<R, K, N, V, 7><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 8: k_batch_phase<R, K, N, V, 8><<<g, kBatchThreads, smem, s>>>(b); break;
-            case 9: k_batch_phase<R, K, N, V, 9><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 0: k_batch_phase<R, K, N, 0><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 1: k_batch_phase<R, K, N, 1><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 2: k_batch_phase<R, K, N, 2><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 3: k_batch_phase<R, K, N, 3><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 4: k_batch_phase<R, K, N, 4><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 5: k_batch_phase<R, K, N, 5><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 6: k_batch_phase<R, K, N, 6><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 7: k_batch_phase<R, K, N, 7><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 8: k_batch_phase<R, K, N, 8><<<g, kBatchThreads, smem, s>>>(b); break;
+            case 9: k_batch_phase<R, K, N, 9><<<g, kBatchThreads, smem, s>>>(b); break;
             default: return cudaErrorInvalidValue;
         }
         return cudaGetLastError();
@@ -68,10 +67,10 @@ template <typename R, typename K, int N, int V> struct BatchLaunch {
 };
 
 // Sizes whose plane does not fit a CTA (128 in FP64 arithmetic) run the tiles of the ten passes.
-template <typename R, typename K, typename F> static bool with_batch_nv(int N, int, F &&f) {
+template <typename R, typename K, typename F> static bool with_tiled(int N, F &&f) {
     if constexpr (!box_fits<R, K, 128>()) {
         if (N == 128) {
-            f(BatchLaunch<R, K, 128, 0>{});
+            f(BatchLaunch<R, K, 128>{});
             return true;
         }
     }
@@ -99,7 +98,7 @@ template <typename R, typename K> struct BatchTable {
             for (int p = 0; p < kBoxPhases; ++p) it[p] = p ? N : 1;
             return true;
         }
-        return with_batch_nv<R, K>(N, 0, [&](auto l) {
+        return with_tiled<R, K>(N, [&](auto l) {
             for (int p = 0; p < kBatchPhases; ++p) it[p] = batch_items<R, K, 128>(p);
             *smem = batch_smem<R, K, 128>();
         });
@@ -140,20 +139,20 @@ template <typename R, typename K> struct BatchTable {
         with_box_nv<R, K>(N, V, [&](auto o) { e = one_phase(o, ph, nb, s, b); });
         return e;
     }
-    static std::string setup(int N, int V, size_t smem, int *fit) {
+    static std::string setup(int N, size_t smem, int *fit) {
         std::string e = "batch: res " + std::to_string(N) + " is not a batch size";
-        with_batch_nv<R, K>(N, V, [&](auto L) { e = decltype(L)::setup(smem, fit); });
+        with_tiled<R, K>(N, [&](auto L) { e = decltype(L)::setup(smem, fit); });
         return e;
     }
-    static cudaError_t persistent(int N, int V, int grid, size_t smem, cudaStream_t s, const BatchArgs &a) {
+    static cudaError_t persistent(int N, int grid, size_t smem, cudaStream_t s, const BatchArgs &a) {
         cudaError_t e = cudaErrorInvalidValue;
-        with_batch_nv<R, K>(N, V, [&](auto L) { e = decltype(L)::persistent(grid, smem, s, a); });
+        with_tiled<R, K>(N, [&](auto L) { e = decltype(L)::persistent(grid, smem, s, a); });
         return e;
     }
-    static cudaError_t phase(int N, int V, int ph, int tiles, int nboxes, size_t smem, cudaStream_t s,
+    static cudaError_t phase(int N, int ph, int tiles, int nboxes, size_t smem, cudaStream_t s,
                              const BatchBox *b) {
         cudaError_t e = cudaErrorInvalidValue;
-        with_batch_nv<R, K>(N, V, [&](auto L) { e = decltype(L)::phase(ph, tiles, nboxes, smem, s, b); });
+        with_tiled<R, K>(N, [&](auto L) { e = decltype(L)::phase(ph, tiles, nboxes, smem, s, b); });
         return e;
     }
     static const BatchKernels &table() {

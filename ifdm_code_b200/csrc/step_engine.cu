@@ -130,9 +130,10 @@ template <typename R_, typename K_, int N> struct Box {
             zt1grid = sms * (b1 > 0 ? b1 : 1);
             zt5grid = sms * (b5 > 0 ? b5 : 1);
             zt9grid = sms * (b9 > 0 ? b9 : 1);
-            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, -1>, ZSM5));
-            CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, +1>, ZSM5));
-            if constexpr (kPairZ) {
+            if constexpr (!kPairZ) {
+                CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, -1>, ZSM5));
+                CUDA_TRY(prep(k_fft_z_tma<N, ZST5, ZB5, R, K, +1>, ZSM5));
+            } else {
                 CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, -1>, ZSM5P));
                 CUDA_TRY(prep(k_fft_z_pair<N, ZST5P, ZB5P, +1>, ZSM5P));
                 CUDA_TRY(prep(k_kick_fft_z_pair<N, ZST1P, ZB1P>, ZSM1P));
