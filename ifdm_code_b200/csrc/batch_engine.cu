@@ -105,8 +105,8 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
             // A cluster of 16 CTAs a box, all steps in one launch, while a CTA has
             // at most two planes and every cluster is resident at once; else a
             // launch per phase over all boxes (group 0).  FP32, us a step, one
-            // against the other: 8 boxes of 32^3 29 / 39, 32 of 48^3 154 / 133,
-            // 2 of 96^3 224 / 110, 64 of 16^3 46 / 38.
+            // against the other: 8 boxes of 32^3 30 / 38, 64 of 16^3 20 / 37, 32 of
+            // 48^3 154 / 133, 2 of 96^3 224 / 110.
             c.group = c.N <= 32 && bk.resident(c.N, 16, true) >= (int)nb ? 16 : 0;
         }
     }

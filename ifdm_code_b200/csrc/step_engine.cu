@@ -210,7 +210,7 @@ template <typename R_, typename K_, int N> struct Box {
     // arithmetic, 128 (8 FP32 or 4 FP64 rows per tile; FP32 at 128 runs the
     // box kernels); ring depth and resident blocks per SM of P1, P5 and P9.
     // D3: one slot (two in P5) and three blocks at 512, six at 256, twelve at
-    // 128: the blocks hide each other's loads (FP64 512^3 step 7.42 -> 7.31 ms
+    // 128: the blocks hide each other's loads (FP64 512^3 step 7.45 -> 7.35 ms
     // against two or three slots at two blocks; 256^3 873 -> 862 us)
     static constexpr bool kZT = (N >= 256 && (std::is_same<R, K>::value || N <= 512)) || (N == 128 && sizeof(K) == 8);
     static constexpr bool D3 = sizeof(C) == 16 && N >= 128 && N <= 512;
@@ -400,10 +400,6 @@ template <typename R_, typename K_, int N> struct Box {
         for (int p = 6; p <= 9; ++p) pass(p, s, nullptr, pw, rhok, ts_adj, nullptr, tw, twh, 0, 0, tm);
     }
 
-    // One axis of a slab's local FFT step (plain passes): axis 2 = z on the
-    // x-slab [planes][N][N], axis 1 = y on the x-slab, axis 0 = x on the
-    // transposed y-slab [N][planes][N] (op 1: forward, -1/(kappa^2 N^3) with
-    // global y offset y0, inverse).
     // Forward pass along axis 1 (y) or 0 (x) of a half spectrum [N][N][NHP]
     // (diagnostics; FP64); a wait that gives up sets ts->err
     static std::string half_axis(G *data, int axis, const C *tw, TState *ts, cudaStream_t s) {
@@ -443,6 +439,10 @@ template <typename R_, typename K_, int N> struct Box {
         }
         return "line_k2 needs FP64";
     }
+    // One axis of a slab's local FFT step (plain passes): axis 2 = z on the
+    // x-slab [planes][N][N], axis 1 = y on the x-slab, axis 0 = x on the
+    // transposed y-slab [N][planes][N] (op 1: forward, -1/(kappa^2 N^3) with
+    // global y offset y0, inverse).
     static std::string fft_slab(G *data, int planes, int axis, int sign, int op, int y0, const C *tw, cudaStream_t s) {
         const size_t nl = size_t(planes) * N;
         if (nl % TL::L || nl % TZ::L) return "planes * n must be a multiple of the tile lines";

@@ -473,9 +473,9 @@ __global__ void __launch_bounds__(ZT<N, R, K>::NT, MINB)
 // two rows, so the density goes from registers straight into the second
 // transform.  The rows of a pair land next to each other in the slot, as the
 // paired loads want them.  Same arithmetic and outputs as k_density_r2c_z_tma,
-// bit for bit.  (Neighbouring rows 2lp and 2lp + 1 in a line share their
-// rounding, which is then coherent over neighbouring rows: density error
-// against FP64 after 1000 steps at 256^3, g = 0, 1.07e-5 against 9.97e-6.)
+// bit for bit.  (Neighbouring rows 2lp and 2lp + 1 in a line are as accurate:
+// density error against FP64 after 1000 steps, two fields at 512^3 and three at
+// 256^3, 1e-6, so / neighbours: 8.4 / 9.2, 7.9 / 7.9; 9.5 / 9.7, 10.6 / 9.4, 9.5 / 9.5.)
 template <int N, int ST, int MINB>
 __global__ void __launch_bounds__(ZT<N>::NT / 2, MINB)
     k_density_r2c_z_pair(float2 *__restrict__ psi, float2 *__restrict__ rhok, TState *__restrict__ ts,
