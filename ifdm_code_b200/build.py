@@ -33,8 +33,11 @@ PER_FILE = {"ic_pipeline.cu": ["--fmad=false"]}
 CXX_FLAGS = ["-O2", "-fPIC", "-std=c++17", "-Wall", "-I" + CSRC, "-I" + INC]
 
 CU_SOURCES = ["step_engine.cu", "batch_engine.cu", "batch_fp64.cu", "batch_fp32.cu", "batch_mixed.cu",
-              "box_fp64.cu", "box_fp32.cu", "box_mixed.cu",
               "ic_pipeline.cu", "static_poisson.cu", "diagnostics.cu"]
+# box_size.cu once per precision mode (storage and arithmetic type) and grid size
+BOX_SIZES = [(name, r, k, n) for name, r, k, sizes in (("fp64", "double", "double", (16, 32, 48, 64, 96)),
+                                                       ("fp32", "float", "float", (16, 32, 48, 64, 96, 128)),
+                                                       ("mixed", "float", "double", (16, 32, 48, 64, 96))) for n in sizes]
 CPP_SOURCES = ["ifdm_api.cpp", "io.cpp", "snapshot_stream.cpp", "ic_stream.cpp"]
 
 
@@ -84,12 +87,15 @@ def build(force: bool = False, verbose: bool = False) -> str:
     hdr = _newest_header()
     jobs = []
     objs = []
-    for s in CU_SOURCES:
+    units = [(s, s, PER_FILE.get(s, [])) for s in CU_SOURCES]
+    units += [("box_size.cu", f"box_{name}_{n}", [f"-DBOX_NAME={name}", f"-DBOX_R={r}", f"-DBOX_K={k}", f"-DBOX_N={n}"])
+              for name, r, k, n in BOX_SIZES]
+    for s, obj, flags in units:
         src = os.path.join(CSRC, s)
-        out = os.path.join(OBJ, s + ".o")
+        out = os.path.join(OBJ, obj + ".o")
         objs.append(out)
         if force or _stale(out, src, hdr):
-            jobs.append([nvcc] + NVCC_FLAGS + PER_FILE.get(s, []) + ["-c", src, "-o", out])
+            jobs.append([nvcc] + NVCC_FLAGS + flags + ["-c", src, "-o", out])
     for s in CPP_SOURCES:
         src = os.path.join(CSRC, s)
         out = os.path.join(OBJ, s + ".o")

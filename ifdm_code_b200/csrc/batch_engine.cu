@@ -87,8 +87,8 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
     for (auto &c : cls_) {
         if (!K_->items(c.N, c.items, &c.smem)) return "batch: res " + std::to_string(c.N) + " is not a batch size";
         const size_t nb = c.boxes.size();
-        const BoxKernels &bk = box_kernels(precision_);
-        c.box = bk.fits(c.N);
+        const BoxKernels *bk = box_kernels(precision_, c.N);
+        c.box = bk != nullptr;
         CUDA_TRY(cudaMalloc(&c.d_boxes, std::max(sizeof(BatchBox), sizeof(BoxRun)) * nb));
         CUDA_TRY(cudaMalloc(&c.d_segs, sizeof(BatchSeg) * nb * kBatchPhases));
         CUDA_TRY(cudaMalloc(&c.d_ctr, sizeof(unsigned long long) * (nb + 1)));
@@ -98,7 +98,7 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
         for (int v = 0; v < 2; ++v) {
             int fit = 0;
             std::string e = c.box ? K_->box_setup(c.N, v) : K_->setup(c.N, c.smem, &fit);
-            if (e.empty() && c.box) e = bk.setup(c.N, v);
+            if (e.empty() && c.box) e = bk->setup(v);
             if (!e.empty()) return e;
         }
         if (c.box) {
@@ -107,7 +107,7 @@ std::string BatchEngine::init(const std::vector<StepEngine *> &boxes, cudaStream
             // launch per phase over all boxes (group 0).  FP32, us a step, one
             // against the other: 8 boxes of 32^3 30 / 38, 64 of 16^3 20 / 37, 32 of
             // 48^3 154 / 133, 2 of 96^3 224 / 110.
-            c.group = c.N <= 32 && bk.resident(c.N, 16, true) >= (int)nb ? 16 : 0;
+            c.group = c.N <= 32 && bk->resident(16, true) >= (int)nb ? 16 : 0;
         }
     }
     CUDA_TRY(cudaMalloc(&d_status_, sizeof(int)));
@@ -230,7 +230,7 @@ std::string BatchEngine::capture_body(int nsteps) {
             l.cluster = true;
             l.stream = c.side;
             for (int n = 0; n < nsteps; n += kBoxLaunchSteps)
-                CUDA_TRY(box_kernels(precision_).run(c.N, V, l, BoxRun{}, (const BoxRun *)c.d_boxes,
+                CUDA_TRY(box_kernels(precision_, c.N)->run(V, l, BoxRun{}, (const BoxRun *)c.d_boxes,
                                                      std::min(kBoxLaunchSteps, nsteps - n)));
         } else if (c.box) {
             for (int s = 0; s < nsteps; ++s)

@@ -1,7 +1,7 @@
 // box_launch.cuh -- host-side launchers of the one-launch box kernels of one
-// precision (box_kernels.cuh), instantiated in box_fp64.cu, box_fp32.cu and
-// box_mixed.cu so they compile in parallel; the engines reach them through
-// the BoxKernels function table.
+// grid size and precision (box_kernels.cuh).  box_size.cu is compiled once for
+// each: they compile in parallel, and a process loads the modules of the sizes it
+// uses (all sizes of a precision in one module took 13-17 ms at its first box).
 #pragma once
 
 #include "box_kernels.cuh"
@@ -21,17 +21,17 @@ struct BoxLaunch {
 };
 
 struct BoxKernels {
-    bool (*fits)(int N);  // a plane of an N-box fits a CTA
-    // set the kernels' attributes on the current device
-    std::string (*setup)(int N, int V);
+    // set the kernels' attributes on the current device; V: radix plan of the run kernel
+    std::string (*setup)(int V);
     // groups of `group` CTAs that are resident at once (a cluster, or a cooperative grid)
-    int (*resident)(int N, int group, bool cluster);
-    cudaError_t (*run)(int N, int V, const BoxLaunch &l, const BoxRun &one, const BoxRun *many, int nsteps);
-    cudaError_t (*load)(int N, const BoxLaunch &l, const BoxRun &one);
-    cudaError_t (*sweep)(int N, const BoxLaunch &l, const BoxSweep &one);
+    int (*resident)(int group, bool cluster);
+    cudaError_t (*run)(int V, const BoxLaunch &l, const BoxRun &one, const BoxRun *many, int nsteps);
+    cudaError_t (*load)(const BoxLaunch &l, const BoxRun &one);
+    cudaError_t (*sweep)(const BoxLaunch &l, const BoxSweep &one);
 };
 
-const BoxKernels &box_kernels(int precision);  // 0 FP64, 1 FP32, 2 mixed
+// precision 0 FP64, 1 FP32, 2 mixed; null where a plane of an N-box does not fit a CTA
+const BoxKernels *box_kernels(int precision, int N);
 
 template <typename R, typename K> struct BoxTable {
     template <typename Fn> static bool with_n(int N, Fn &&f) {
@@ -51,30 +51,12 @@ template <typename R, typename K> struct BoxTable {
             default: return false;
         }
     }
-    // f(kernel, threads, shared memory) of the run kernel with plan V
-    template <typename Fn> static bool with_run(int N, int V, Fn &&f) {
-        if (!V) return with_n(N, [&](auto o) { pass_run<0>(o, f); });
-        switch (N) {
-            case 32: pass_run<1>(BoxOps<R, K, 32, 1>{}, f); return true;
-            case 48: pass_run<1>(BoxOps<R, K, 48, 1>{}, f); return true;
-            case 64: pass_run<1>(BoxOps<R, K, 64, 1>{}, f); return true;
-            case 96: pass_run<1>(BoxOps<R, K, 96, 1>{}, f); return true;
-            default: return with_n(N, [&](auto o) { pass_run<0>(o, f); });
-        }
-    }
-    template <int V, typename RR, typename KK, int N, int V2, typename Fn>
-    static void pass_run(BoxOps<RR, KK, N, V2>, Fn &&f) {
-        using O = BoxOps<RR, KK, N, V2>;
-        f(k_box_run<RR, KK, N, V2>, int(O::NT), size_t(O::SMEM));
-    }
-    template <typename RR, typename KK, int N, int V2, typename Fn> static void pass_load(BoxOps<RR, KK, N, V2>, Fn &&f) {
-        using O = BoxOps<RR, KK, N, V2>;
-        f(k_box_load<RR, KK, N, V2>, int(O::NT), size_t(O::SMEM));
-    }
-    template <typename RR, typename KK, int N, int V2, typename Fn> static void pass_sweep(BoxOps<RR, KK, N, V2>, Fn &&f) {
-        using O = BoxOps<RR, KK, N, V2>;
-        f(k_box_sweep<RR, KK, N, V2>, int(O::NT), size_t(O::SMEM));
-    }
+};
+
+template <typename R, typename K, int N> struct BoxSize {
+    using O = BoxOps<R, K, N, 0>;
+    // another radix plan (V = 1)
+    static constexpr bool kTwoPlans = N != 16 && N != 128;
 
     template <typename Kern> static cudaError_t attributes(Kern k, size_t smem) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -100,88 +82,73 @@ template <typename R, typename K> struct BoxTable {
         c->numAttrs = 1;
     }
 
-    static bool fits(int N) {
-        return with_n(N, [](auto) {});
-    }
-    static std::string setup(int N, int V) {
-        cudaError_t e = cudaErrorInvalidValue;
-        with_run(N, V, [&](auto k, int, size_t smem) { e = attributes(k, smem); });
-        if (e == cudaSuccess && !V)
-            with_n(N, [&](auto o) {
-                pass_load(o, [&](auto k, int, size_t smem) { e = attributes(k, smem); });
-                if (e == cudaSuccess) pass_sweep(o, [&](auto k, int, size_t smem) { e = attributes(k, smem); });
-            });
+    static std::string setup(int V) {
+        cudaError_t e = cudaSuccess;
+        if constexpr (kTwoPlans) {
+            if (V) e = attributes(k_box_run<R, K, N, 1>, BoxOps<R, K, N, 1>::SMEM);
+        }
+        if (!V || !kTwoPlans) {
+            e = attributes(k_box_run<R, K, N, 0>, O::SMEM);
+            if (e == cudaSuccess) e = attributes(k_box_load<R, K, N, 0>, O::SMEM);
+            if (e == cudaSuccess) e = attributes(k_box_sweep<R, K, N, 0>, O::SMEM);
+        }
         return e == cudaSuccess ? "" : std::string("box kernel setup: ") + cudaGetErrorString(e);
     }
-    static int resident(int N, int group, bool cluster) {
-        int best = 1 << 30;
-        auto one = [&](auto k, int nt, size_t smem) {
-            int n = 0;
-            if (cluster) {
-                BoxLaunch l;
-                l.group = group;
-                l.cluster = true;
-                cudaLaunchConfig_t c;
-                cudaLaunchAttribute at;
-                config(l, nt, smem, &c, &at);
-                if (cudaOccupancyMaxActiveClusters(&n, k, &c) != cudaSuccess) n = 0;
-            } else {
-                int dev = 0, sms = 0, per = 0, coop = 0;
-                if (cudaGetDevice(&dev) != cudaSuccess ||
-                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-                    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, nt, smem) != cudaSuccess)
-                    per = sms = 0;
-                n = per * sms / group;
-            }
-            if (n < best) best = n;
-        };
-        cudaGetLastError();
-        if (!with_n(N, [&](auto o) {
-                pass_run<0>(o, one);
-                pass_load(o, one);
-                pass_sweep(o, one);
-            }))
-            return 0;
-        cudaGetLastError();
-        return best;
-    }
-    static cudaError_t run(int N, int V, const BoxLaunch &l, const BoxRun &one, const BoxRun *many, int nsteps) {
-        cudaError_t e = cudaErrorInvalidValue;
-        with_run(N, V, [&](auto k, int nt, size_t smem) {
+    template <typename Kern> static int resident_of(Kern k, int group, bool cluster) {
+        int n = 0;
+        if (cluster) {
+            BoxLaunch l;
+            l.group = group;
+            l.cluster = true;
             cudaLaunchConfig_t c;
             cudaLaunchAttribute at;
-            config(l, nt, smem, &c, &at);
-            e = cudaLaunchKernelEx(&c, k, one, many, nsteps, l.group, int(l.cluster));
-        });
-        return e;
+            config(l, O::NT, O::SMEM, &c, &at);
+            if (cudaOccupancyMaxActiveClusters(&n, k, &c) != cudaSuccess) n = 0;
+        } else {
+            int dev = 0, sms = 0, per = 0, coop = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, O::NT, O::SMEM) != cudaSuccess)
+                per = sms = 0;
+            n = per * sms / group;
+        }
+        return n;
     }
-    static cudaError_t load(int N, const BoxLaunch &l, const BoxRun &one) {
-        cudaError_t e = cudaErrorInvalidValue;
-        with_n(N, [&](auto o) {
-            pass_load(o, [&](auto k, int nt, size_t smem) {
-                cudaLaunchConfig_t c;
-                cudaLaunchAttribute at;
-                config(l, nt, smem, &c, &at);
-                e = cudaLaunchKernelEx(&c, k, one, l.group, int(l.cluster));
-            });
-        });
-        return e;
+    static int resident(int group, bool cluster) {
+        cudaGetLastError();
+        const int n[3] = {resident_of(k_box_run<R, K, N, 0>, group, cluster), resident_of(k_box_load<R, K, N, 0>, group, cluster),
+                          resident_of(k_box_sweep<R, K, N, 0>, group, cluster)};
+        cudaGetLastError();
+        return n[0] < n[1] ? (n[0] < n[2] ? n[0] : n[2]) : (n[1] < n[2] ? n[1] : n[2]);
     }
-    static cudaError_t sweep(int N, const BoxLaunch &l, const BoxSweep &one) {
-        cudaError_t e = cudaErrorInvalidValue;
-        with_n(N, [&](auto o) {
-            pass_sweep(o, [&](auto k, int nt, size_t smem) {
-                cudaLaunchConfig_t c;
-                cudaLaunchAttribute at;
-                config(l, nt, smem, &c, &at);
-                e = cudaLaunchKernelEx(&c, k, one, l.group, int(l.cluster));
-            });
-        });
-        return e;
+    template <int V> static cudaError_t run_plan(const BoxLaunch &l, const BoxRun &one, const BoxRun *many, int nsteps) {
+        using P = BoxOps<R, K, N, V>;
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute at;
+        config(l, P::NT, P::SMEM, &c, &at);
+        return cudaLaunchKernelEx(&c, k_box_run<R, K, N, V>, one, many, nsteps, l.group, int(l.cluster));
+    }
+    static cudaError_t run(int V, const BoxLaunch &l, const BoxRun &one, const BoxRun *many, int nsteps) {
+        if constexpr (kTwoPlans) {
+            if (V) return run_plan<1>(l, one, many, nsteps);
+        }
+        return run_plan<0>(l, one, many, nsteps);
+    }
+    static cudaError_t load(const BoxLaunch &l, const BoxRun &one) {
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute at;
+        config(l, O::NT, O::SMEM, &c, &at);
+        return cudaLaunchKernelEx(&c, k_box_load<R, K, N, 0>, one, l.group, int(l.cluster));
+    }
+    static cudaError_t sweep(const BoxLaunch &l, const BoxSweep &one) {
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute at;
+        config(l, O::NT, O::SMEM, &c, &at);
+        return cudaLaunchKernelEx(&c, k_box_sweep<R, K, N, 0>, one, l.group, int(l.cluster));
     }
     static const BoxKernels &table() {
-        static const BoxKernels t{&fits, &setup, &resident, &run, &load, &sweep};
+        static const BoxKernels t{&setup, &resident, &run, &load, &sweep};
         return t;
     }
 };

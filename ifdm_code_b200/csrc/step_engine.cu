@@ -631,11 +631,25 @@ static std::string get_twiddles(int n, int prec, void **out) {
     return "";
 }
 
-const BoxKernels &box_kernels_fp64();
-const BoxKernels &box_kernels_fp32();
-const BoxKernels &box_kernels_mixed();
-const BoxKernels &box_kernels(int precision) {
-    return precision == 0 ? box_kernels_fp64() : precision == 1 ? box_kernels_fp32() : box_kernels_mixed();
+#define BOX_SIZES(X, name) X(name, 16) X(name, 32) X(name, 48) X(name, 64) X(name, 96)
+#define BOX_DECLARE(name, n) const BoxKernels &box_kernels_##name##_##n();
+#define BOX_CASE(name, n) \
+    case n: return &box_kernels_##name##_##n();
+BOX_SIZES(BOX_DECLARE, fp64)
+BOX_SIZES(BOX_DECLARE, fp32)
+BOX_DECLARE(fp32, 128)
+BOX_SIZES(BOX_DECLARE, mixed)
+static_assert(box_fits<float, float, 128>() && !box_fits<double, double, 128>() && !box_fits<float, double, 128>(), "sizes");
+
+const BoxKernels *box_kernels(int precision, int N) {
+    if (precision == 0) {
+        switch (N) { BOX_SIZES(BOX_CASE, fp64) }
+    } else if (precision == 1) {
+        switch (N) { BOX_SIZES(BOX_CASE, fp32) BOX_CASE(fp32, 128) }
+    } else {
+        switch (N) { BOX_SIZES(BOX_CASE, mixed) }
+    }
+    return nullptr;
 }
 
 // ------------------------------------------------------------ StepEngine --
@@ -732,8 +746,8 @@ std::string StepEngine::init(const EngineConfig &cfg, cudaStream_t stream) {
 // IFDM_NO_FUSE keeps the one-launch-per-pass kernels.
 std::string StepEngine::init_box() {
     const int N = cfg_.N;
-    const BoxKernels &bk = box_kernels(cfg_.precision);
-    if (!bk.fits(N)) return "";
+    const BoxKernels *bk = box_kernels(cfg_.precision, N);
+    if (!bk) return "";
     // one CTA per plane; a cluster where that is a cluster (its barrier takes
     // 1000-2000 cycles against 3000 of the counter in global memory), else a cooperative grid
     box_group_ = N;
@@ -748,9 +762,9 @@ std::string StepEngine::init_box() {
         const std::array<int, 3> key{dev, N, cfg_.precision};
         auto it = known.find(key);
         if (it == known.end()) {
-            std::string e = bk.setup(N, 0);
+            std::string e = bk->setup(0);
             if (!e.empty()) return e;
-            it = known.emplace(key, bk.resident(N, box_group_, box_cluster_)).first;
+            it = known.emplace(key, bk->resident(box_group_, box_cluster_)).first;
         }
         resident = it->second;
     }
@@ -856,7 +870,7 @@ std::string StepEngine::box_run(int nsteps, int timestep, double dt_scale, void 
         a.log = log ? (StepLog *)log + n : nullptr;
         a.seg_psi = save ? (char *)seg_psi_ + size_t(n) * n3 * 2 * rs : nullptr;
         a.seg_phi = save ? (char *)seg_phi_ + size_t(n) * n3 * rs : nullptr;
-        CUDA_TRY(box_kernels(cfg_.precision).run(cfg_.N, 0, l, a, nullptr, cnt));
+        CUDA_TRY(box_kernels(cfg_.precision, cfg_.N)->run(0, l, a, nullptr, cnt));
     }
     return "";
 }
@@ -954,7 +968,7 @@ std::string StepEngine::load_psi(const double *psi, bool on_device, double a, do
         l.cluster = box_cluster_;
         l.stream = stream_;
         CUDA_TRY(cudaMemsetAsync(box_scr_, 0, sizeof(BoxScratch), stream_));
-        CUDA_TRY(box_kernels(prec).load(cfg_.N, l, a0));
+        CUDA_TRY(box_kernels(prec, cfg_.N)->load(l, a0));
     } else {
         std::string e = launch_initial_density();
         if (!e.empty()) return e;
@@ -1372,13 +1386,13 @@ std::string StepEngine::adjoint_box(const TState &fin) {
     l.group = box_group_;
     l.cluster = box_cluster_;
     l.stream = stream_;
-    const BoxKernels &bk = box_kernels(cfg_.precision);
+    const BoxKernels &bk = *box_kernels(cfg_.precision, cfg_.N);
     // the output map: psi_out = S psi exp(-i (pendP phi + pendQ |psi|^2 - gphase))
     a.start = a.end = M;
     a.a = fin.pendP;
     a.b = fin.pendQ;
     a.alpha = -fin.gphase;
-    CUDA_TRY(bk.sweep(cfg_.N, l, a));
+    CUDA_TRY(bk.sweep(l, a));
     for (int seg = (M - 1) / K; seg >= 0; --seg) {
         const int start = seg * K, end = std::min(M, start + K);
         CUDA_TRY(cudaMemcpyAsync(psi_, (char *)ckpt_psi_ + size_t(seg) * n3 * cs, n3 * cs, cudaMemcpyDeviceToDevice,
@@ -1391,7 +1405,7 @@ std::string StepEngine::adjoint_box(const TState &fin) {
         }
         a.start = start;
         a.end = end;
-        CUDA_TRY(bk.sweep(cfg_.N, l, a));
+        CUDA_TRY(bk.sweep(l, a));
     }
     return "";
 }
